@@ -16,9 +16,11 @@ from . import _lib
 def _check_inputs(a, b, a_scale, b_scale, c):
     if not (a.is_cuda and b.is_cuda and a_scale.is_cuda and b_scale.is_cuda and c.is_cuda):
         raise ValueError("fp8_mm: all tensors must be CUDA tensors (there is no CPU path)")
-    for name, t in (("a", a), ("b", b), ("a_scale", a_scale), ("b_scale", b_scale), ("c", c)):
-        if not t.is_contiguous():
-            raise ValueError(f"fp8_mm: {name} must be contiguous (K-major layout)")
+    if not (a.is_contiguous() and b.is_contiguous() and a_scale.is_contiguous() and b_scale.is_contiguous()
+            and c.is_contiguous()):
+        for name, t in (("a", a), ("b", b), ("a_scale", a_scale), ("b_scale", b_scale), ("c", c)):
+            if not t.is_contiguous():
+                raise ValueError(f"fp8_mm: {name} must be contiguous (K-major layout)")
     if a.element_size() != 1 or b.element_size() != 1:
         raise ValueError("fp8_mm: a and b must be 1-byte e4m3 tensors")
     if a_scale.dtype != torch.float32 or b_scale.dtype != torch.float32:
@@ -45,7 +47,7 @@ def fp8_mm(a, b, a_scale, b_scale, c, split_k: int = 0, workspace=None):
     """
     m, n, k = _check_inputs(a, b, a_scale, b_scale, c)
     L = _lib.lib()
-    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    stream = _lib.current_stream()
     if workspace is None and split_k == 0:
         L.run(a.data_ptr(), b.data_ptr(), a_scale.data_ptr(), b_scale.data_ptr(), c.data_ptr(), m, n, k, None, stream)
         return c
@@ -92,7 +94,7 @@ def fp8_mm_reference_layout(a, b, a_scale, b_scale, c, fnuz=None):
         if (b.dtype == torch.float8_e4m3fnuz) != fnuz:
             raise ValueError("fp8_mm_reference_layout: a and b must use the same FP8 format")
     L = _lib.lib()
-    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    stream = _lib.current_stream()
     entry = L.rf_fp8_gemm_colmajor_fnuz if fnuz else L.rf_fp8_gemm_colmajor
     st = entry(a.data_ptr(), b.data_ptr(), a_scale.data_ptr(), b_scale.data_ptr(), c.data_ptr(), m, n, k, None, 0,
                stream)

@@ -7,6 +7,7 @@ dict).  Unlike the reference wrapper, the router matmul also runs in the library
 not in PyTorch.  All tensors must be contiguous CUDA fp16 tensors; there is no CPU path.
 """
 import ctypes
+import functools
 
 import torch
 
@@ -37,6 +38,26 @@ def _check_fp16_cuda(name, t):
         raise ValueError(f"moe: {name} must be a contiguous CUDA fp16 tensor (there is no CPU path)")
 
 
+@functools.lru_cache(maxsize=None)
+def _expert_names(n_experts, j):
+    return tuple(f"experts.{i}.{j}.weight" for i in range(n_experts))
+
+
+def _expert_ptrs(weights, n_experts, j, ctype):
+    """ctypes array of the addresses of matrix `j` (0 gate, 1 up, 2 down) of every expert.
+
+    A layer of 32 experts has 96 of these tensors and nothing is enqueued before their addresses are known, so the
+    loop does no more than it must: names made once per expert count, one condition per tensor.
+    """
+    ts = [weights[name] for name in _expert_names(n_experts, j)]
+    f16 = torch.float16
+    for t in ts:
+        if not (t.is_cuda and t.dtype is f16 and t.is_contiguous()):
+            for name, u in zip(_expert_names(n_experts, j), ts):
+                _check_fp16_cuda(name, u)
+    return (ctype * n_experts)(*[t.data_ptr() for t in ts])
+
+
 class MoEBuffers:
     """A filled MoEInputRaw (src/moe/moe.h:14-65) plus the torch tensors that own its buffers."""
 
@@ -53,14 +74,7 @@ class MoEBuffers:
         raw.params = _lib.InputParams(int(config.get("batch_size", 1)), T // int(config.get("batch_size", 1)), d, f,
                                       E, K, ns, 0)
         self._keep = [x, weights]
-        arrs = []
-        for j in range(3):
-            arr = (ctypes.c_void_p * E)()
-            for i in range(E):
-                w = weights[f"experts.{i}.{j}.weight"]
-                _check_fp16_cuda(f"experts.{i}.{j}.weight", w)
-                arr[i] = w.data_ptr()
-            arrs.append(arr)
+        arrs = [_expert_ptrs(weights, E, j, ctypes.c_void_p) for j in range(3)]
         self._keep.append(arrs)
         raw.expert_weight_gate = ctypes.cast(arrs[0], ctypes.POINTER(ctypes.c_void_p))
         raw.expert_weight_up = ctypes.cast(arrs[1], ctypes.POINTER(ctypes.c_void_p))
@@ -95,7 +109,7 @@ def moe_forward(x, weights, config, expert_scores=None, router_bias=None, metric
     """
     L = _lib.lib()
     buf = MoEBuffers(x, weights, config, expert_scores)
-    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    stream = _lib.current_stream()
     pm = ctypes.byref(metrics) if metrics is not None else None
     if expert_scores is not None:
         st = L.run_topk(ctypes.byref(buf.raw), stream, pm)
@@ -130,15 +144,7 @@ def custom_kernel(data):
     L = _lib.lib()
     E = int(config["n_routed_experts"])
     out = torch.empty_like(x)
-    ull = ctypes.c_ulonglong
-    ptrs = []
-    for j in range(3):
-        arr = (ull * E)()
-        for i in range(E):
-            w = weights[f"experts.{i}.{j}.weight"]
-            _check_fp16_cuda(f"experts.{i}.{j}.weight", w)
-            arr[i] = w.data_ptr()
-        ptrs.append(arr)
+    ptrs = [_expert_ptrs(weights, E, j, ctypes.c_ulonglong) for j in range(3)]
     sh = [weights[f"shared_experts.{j}.weight"] for j in range(3)]
     for j, w in enumerate(sh):
         _check_fp16_cuda(f"shared_experts.{j}.weight", w)
@@ -149,6 +155,6 @@ def custom_kernel(data):
         seq, bs, int(config["d_hidden"]), int(config["d_expert"]), E, int(config["n_experts_per_token"]),
         int(config["n_shared_experts"]), x.data_ptr(), 0, ptrs[0], ptrs[1], ptrs[2], sh[0].data_ptr(),
         sh[1].data_ptr(), sh[2].data_ptr(), weights["router.weight"].data_ptr(), out.data_ptr(),
-        ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+        _lib.current_stream())
     _lib.check(st, "rf_run_from_python")
     return out

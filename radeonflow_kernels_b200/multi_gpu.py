@@ -145,7 +145,7 @@ def stream_barrier(flag: torch.Tensor, group=None):
 
 
 def _stream():
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return _lib.current_stream()
 
 
 # --------------------------------------------------------------------------------- N-split GEMM --
