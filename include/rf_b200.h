@@ -339,10 +339,11 @@ int rf_moe_grouped_gemm(const void *x, int n_rows, const void *const *w_ptrs_hos
  * (hipBLASLt takes raw pointers, src/moe/gemm_thirdparty.cpp:65-115).                               */
 int rf_moe_set_map_cache_sets(int max_sets);
 
-/* on != 0: rf_moe_forward and rf_run_from_python let the first expert GEMM gather the token rows in its
- * own loader (expand_input, src/moe/moe_topk_kernel.cpp:174-213, fused) and leave expanded_seq_input
- * unwritten; run_topk always writes it, as the reference's checker expects.  Same bits either way.  Off by
- * default (RF_MOE_FUSED_GATHER=1 turns it on at first use): measured, the separate gather pass is faster.  */
+/* on != 0: rf_moe_forward and rf_run_from_python leave expanded_seq_input (expand_input's output,
+ * src/moe/moe_topk_kernel.cpp:174-213) unwritten: the token rows of the experts pass through
+ * expanded_fc2_output, before fc2 writes its results there.  run_topk always writes expanded_seq_input, as the
+ * reference's checker expects.  Same bits and the same speed either way.  Off by default (RF_MOE_FUSED_GATHER=1
+ * turns it on at first use).                                                                            */
 int rf_moe_set_fused_gather(int on);
 
 /* Grid cap of the grouped GEMMs that THIS host thread enqueues from now on (0 = one persistent CTA per SM,

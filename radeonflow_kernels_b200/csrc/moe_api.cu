@@ -33,7 +33,7 @@ int validate_params(const InputParams& q) {
 // ---------------------------------------------------------------- per-expert tensor-map cache --
 // Weights are static across calls, so the device array of tensor maps built for a set of weight
 // pointers is kept and found again by (device, pointers, shape).  The cache holds 2048 sets by default (a
-// model of 100 MoE layers uses about 700) and evicts the least recently used one; a set used by the
+// model of 100 MoE layers uses about 300) and evicts the least recently used one; a set used by the
 // grouped GEMM that is being enqueued is never evicted, and an evicted array is freed only after an event
 // recorded on the calling stream has completed, so a kernel that was enqueued with it can still read it.
 // (That, like the shared tile-list scratch, assumes what the reference also assumes: the MoE entry points
@@ -136,35 +136,24 @@ thread_local int g_grid_limit = 0;
 
 // ------------------------------------------------------------------------------ aux scratch --
 struct Aux {
-    int* tile_group;
-    int* tile_row0;
-    int* tile_chunk;
-    int* tile_count;
-    int* single_offsets;   // [2] = {0, T} for the shared expert / router (one group)
+    rf::MoeTile* tiles;
+    int* counters;         // moe_tile_list_launch
     int* sort_scratch;
 };
 
-size_t aux_bytes(int n_rows_expanded, int n_experts) {
-    const size_t max_tiles = (size_t)n_rows_expanded / 128 + n_experts + 2;
-    return align_up(max_tiles * 4, 256) * 3 + 256 + 256 +
-           align_up(rf::moe_permute_scratch_bytes(n_rows_expanded, n_experts), 256);
+// row tiles of `rows` expanded rows in n_groups groups and of n_alt rows of the alt group
+size_t max_tiles(int rows, int n_groups, int n_alt) {
+    return (size_t)rows / rf::kMoeTileRows + n_groups + (size_t)n_alt / rf::kMoeTileRows + 2;
 }
 
-bool carve_aux(Aux* a, int n_rows_expanded, int n_experts) {
-    const size_t max_tiles = (size_t)n_rows_expanded / 128 + n_experts + 2;
-    char* base = static_cast<char*>(rf::device_scratch(aux_bytes(n_rows_expanded, n_experts), rf::kScratchMoeAux));
+bool carve_aux(Aux* a, int rows, int n_groups, int n_alt) {
+    const size_t tile_bytes = align_up(max_tiles(rows, n_groups, n_alt) * sizeof(rf::MoeTile), 256);
+    const size_t sort_bytes = align_up(rf::moe_permute_scratch_bytes(rows, n_groups), 256);
+    char* base = static_cast<char*>(rf::device_scratch(tile_bytes + 256 + sort_bytes, rf::kScratchMoeAux));
     if (!base) return false;
-    a->tile_group = reinterpret_cast<int*>(base);
-    base += align_up(max_tiles * 4, 256);
-    a->tile_row0 = reinterpret_cast<int*>(base);
-    base += align_up(max_tiles * 4, 256);
-    a->tile_chunk = reinterpret_cast<int*>(base);
-    base += align_up(max_tiles * 4, 256);
-    a->tile_count = reinterpret_cast<int*>(base);
-    base += 256;
-    a->single_offsets = reinterpret_cast<int*>(base);
-    base += 256;
-    a->sort_scratch = reinterpret_cast<int*>(base);
+    a->tiles = reinterpret_cast<rf::MoeTile*>(base);
+    a->counters = reinterpret_cast<int*>(base + tile_bytes);
+    a->sort_scratch = reinterpret_cast<int*>(base + tile_bytes + 256);
     return true;
 }
 
@@ -209,73 +198,107 @@ struct StageTimer {
     }
 };
 
-// One grouped GEMM: rows of `x` [n_rows, k] by per-group weights; `offsets_dev` has n_groups+1 entries.
-int grouped_gemm(int mode, const void* x, int n_rows, const void* const* w_host, const void* const* w2_host,
-                 int n_groups, const int* offsets_dev, int n_out, int k, const float* bias, void* out, const Aux& aux,
-                 DeviceState* st, cudaStream_t stream, const int* scatter_meta = nullptr,
-                 const rf::PeerPtrs* scatter_dst = nullptr, const int* gather_map = nullptr, int gather_mod = 0) {
-    if (n_rows <= 0) return RF_OK;
-    const CUtensorMap* maps;
-    const CUtensorMap* maps2 = nullptr;
+// Rows of the alt group of a grouped GEMM (the shared expert): `rows` rows of x [rows, k], results in out.
+struct AltGroup {
+    const void* x = nullptr;
+    int rows = 0;
+    void* out = nullptr;
+};
+
+// Result rows stored through a table of return addresses instead of in order.
+struct RowScatter {
+    const int* meta = nullptr;
+    const rf::PeerPtrs* dst = nullptr;
+};
+
+bool encode_row_maps(rf::MoeRowMaps* m, const void* x, int rows, int k) {
+    uint32_t box_rows = 16;
+    for (CUtensorMap& map : m->box) {
+        if (!rf::encode_tma_2d(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, x, (uint64_t)rows, (uint64_t)k,
+                               (uint64_t)k * 2, box_rows, 64, true))
+            return false;
+        box_rows += 16;
+    }
+    return true;
+}
+
+int build_tiles(const int* offsets_dev, int n_groups, int alt_rows, const Aux& aux, cudaStream_t stream) {
+    return rf::moe_tile_list_launch(offsets_dev, n_groups, alt_rows, aux.tiles, aux.counters, stream) == cudaSuccess
+               ? RF_OK : RF_ERR_CUDA;
+}
+
+// The `nth` grouped GEMM (< kMoeItemCounters) over the row tiles built last in `aux`: rows of `x` [n_rows, k] by per-group weights (w2_host: SwiGLU of the
+// two products).  With alt.rows > 0 the weight lists hold one entry more, the alt group's, behind the n_groups others.
+int grouped_gemm(int nth, const void* x, int n_rows, const void* const* w_host, const void* const* w2_host, int n_groups,
+                 int n_out, int k, void* out, const Aux& aux, DeviceState* st, cudaStream_t stream,
+                 const AltGroup& alt = {}, const RowScatter& scatter = {}) {
+    if (n_rows <= 0 && alt.rows <= 0) return RF_OK;
+    // result rows leave as 16-byte stores
+    if (((uintptr_t)out | (uintptr_t)alt.out) & 15) return RF_ERR_CUDA;
+    const int n_sets = n_groups + (alt.rows > 0 ? 1 : 0);
     begin_map_call();
-    if (mode == rf::kMoeGemmRouter) {
-        maps = weight_maps(w_host, 1, n_out, k, 256, 64, stream);            // [N, K] row-major, box 256 rows x 64 K
-    } else {
-        maps = weight_maps(w_host, n_groups, k, n_out, 64, 64, stream);      // [K, N] row-major, box 64 K-rows x 64 N
-        if (mode == rf::kMoeGemmSwiglu) maps2 = weight_maps(w2_host, n_groups, k, n_out, 64, 64, stream);
-    }
-    if (!maps || (mode == rf::kMoeGemmSwiglu && !maps2)) return RF_ERR_CUDA;
-    // with a row map `x` is the token matrix [gather_mod, k], read row by row by the kernel's gather warps (the
-    // A tensor map is then not used, but stays a valid one)
-    if (gather_map && (mode != rf::kMoeGemmSwiglu || gather_mod <= 0)) return RF_ERR_UNSUPPORTED;
-    CUtensorMap ta, to;
-    if (!rf::encode_tma_2d(&ta, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, x, (uint64_t)(gather_map ? gather_mod : n_rows),
-                           (uint64_t)k, (uint64_t)k * 2, 128, 64, true))
-        return RF_ERR_CUDA;
-    const bool tma_store = (n_out % 64) == 0 && !scatter_meta;
-    if (tma_store) {
-        if (!rf::encode_tma_2d(&to, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, out, (uint64_t)n_rows, (uint64_t)n_out,
-                               (uint64_t)n_out * 2, 32, 64, true))
-            return RF_ERR_CUDA;
-    } else {
-        to = ta;
-    }
-    if (rf::moe_tile_list_launch(offsets_dev, n_groups, aux.tile_group, aux.tile_row0, aux.tile_chunk, aux.tile_count, stream) !=
-        cudaSuccess)
-        return RF_ERR_CUDA;
+    // [K, N] row-major, box 64 K-rows x 64 N
+    const CUtensorMap* maps = weight_maps(w_host, n_sets, k, n_out, 64, 64, stream);
+    const CUtensorMap* maps2 = w2_host ? weight_maps(w2_host, n_sets, k, n_out, 64, 64, stream) : nullptr;
+    if (!maps || (w2_host && !maps2)) return RF_ERR_CUDA;
+    rf::MoeRowMaps mx, ma;
+    if (n_rows > 0 && !encode_row_maps(&mx, x, n_rows, k)) return RF_ERR_CUDA;
+    if (alt.rows > 0 && !encode_row_maps(&ma, alt.x, alt.rows, k)) return RF_ERR_CUDA;
+    if (alt.rows <= 0) ma = mx;
+    if (n_rows <= 0) mx = ma;
     rf::MoeGemmParams p;
-    p.tile_group = aux.tile_group;
-    p.tile_row0 = aux.tile_row0;
-    p.tile_chunk = aux.tile_chunk;
-    p.tile_count = aux.tile_count;
-    p.group_offsets = offsets_dev;
-    p.b_maps = maps;
-    p.b2_maps = maps2;
-    p.bias = bias;
+    p.tiles = aux.tiles;
+    p.tile_count = aux.counters;
+    p.next_item = aux.counters + 1 + nth;
+    p.w_maps = maps;
+    p.w2_maps = maps2;
     p.out = out;
+    p.alt_group = alt.rows > 0 ? n_groups : -1;
+    p.alt_out = alt.out;
     p.n_out = n_out;
     p.k = k;
-    p.tma_store = tma_store ? 1 : 0;
-    p.gather_src = gather_map ? x : nullptr;
-    p.gather_map = gather_map;
-    p.gather_mod = gather_mod;
-    p.gather_rows = n_rows;
-    p.scatter_meta = scatter_meta;
-    if (scatter_dst) p.scatter_dst = *scatter_dst;
+    p.scatter_meta = scatter.meta;
+    if (scatter.dst) p.scatter_dst = *scatter.dst;
     else memset(&p.scatter_dst, 0, sizeof p.scatter_dst);
     p.status = st->status;
     p.launch_tag = rf::next_launch_tag();
     const int ctas = g_grid_limit > 0 && g_grid_limit < st->num_sms ? g_grid_limit : st->num_sms;
-    if (rf::moe_gemm_launch(mode, ta, to, p, ctas, stream) != cudaSuccess) return RF_ERR_CUDA;
-    return RF_OK;
+    return rf::moe_gemm_launch(w2_host != nullptr, mx, ma, p, ctas, stream) == cudaSuccess ? RF_OK : RF_ERR_CUDA;
 }
 
-int set_single_offsets(const Aux& aux, int n_rows, cudaStream_t stream) {
-    return rf::moe_set_range_launch(aux.single_offsets, 0, n_rows, stream) == cudaSuccess ? RF_OK : RF_ERR_CUDA;
+// logits [n_rows, n_out] = x [n_rows, k] . w [n_out, k]^T + bias
+int router_gemm(const void* x, const void* w, const float* bias, int n_rows, int n_out, int k, void* out,
+                DeviceState* st, cudaStream_t stream) {
+    CUtensorMap tx, tw, to;
+    if (((uintptr_t)w & 15) ||
+        !rf::encode_tma_2d(&tx, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, x, (uint64_t)n_rows, (uint64_t)k, (uint64_t)k * 2,
+                           128, 64, true) ||
+        !rf::encode_tma_2d(&tw, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, w, (uint64_t)n_out, (uint64_t)k, (uint64_t)k * 2,
+                           256, 64, true))
+        return RF_ERR_CUDA;
+    rf::MoeRouterParams p;
+    p.tma_store = n_out % 64 == 0;
+    if (p.tma_store) {
+        if (!rf::encode_tma_2d(&to, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, out, (uint64_t)n_rows, (uint64_t)n_out,
+                               (uint64_t)n_out * 2, 32, 64, true))
+            return RF_ERR_CUDA;
+    } else {
+        to = tx;
+    }
+    p.bias = bias;
+    p.out = out;
+    p.n_rows = n_rows;
+    p.n_out = n_out;
+    p.k = k;
+    p.status = st->status;
+    p.launch_tag = rf::next_launch_tag();
+    const int ctas = g_grid_limit > 0 && g_grid_limit < st->num_sms ? g_grid_limit : st->num_sms;
+    return rf::moe_router_launch(tx, tw, to, p, ctas, stream) == cudaSuccess ? RF_OK : RF_ERR_CUDA;
 }
 
-// `fill_expanded`: write expanded_seq_input (the reference's expand_input output, a stage tensor its checker
-// compares) and let fc1 read it; false: fc1 gathers the token rows itself and the buffer is left untouched.
+// `fill_expanded`: the gathered token rows go to expanded_seq_input (the reference's expand_input output, a stage
+// tensor its checker compares); false: that buffer is left untouched and the rows pass through expanded_fc2_output,
+// which has their size and is first written by fc2.
 int moe_layer(MoEInputRaw* in, bool compute_router, const float* router_bias, cudaStream_t stream,
               PerfMetrics* metrics, bool fill_expanded) {
     if (!in) return RF_ERR_NULL_POINTER;
@@ -298,17 +321,14 @@ int moe_layer(MoEInputRaw* in, bool compute_router, const float* router_bias, cu
     DeviceState* st = rf::device_state();
     if (!st) return RF_ERR_CUDA;
     Aux aux;
-    if (!carve_aux(&aux, TK > T ? TK : T, E)) return RF_ERR_CUDA;
+    if (!carve_aux(&aux, TK, E, T)) return RF_ERR_CUDA;
 
     StageTimer tm(metrics, stream);
     const int t_begin = tm.mark();
-    if ((rc = set_single_offsets(aux, T, stream)) != RF_OK) return rc;
 
     // ---- router GEMM (optional), softmax + top-k, counting sort, row gather  -> "moe_misc"
     if (compute_router) {
-        const void* rw[1] = {in->router_weight};
-        rc = grouped_gemm(rf::kMoeGemmRouter, in->input_seq, T, rw, nullptr, 1, aux.single_offsets, E, d, router_bias,
-                          in->expert_scores, aux, st, stream);
+        rc = router_gemm(in->input_seq, in->router_weight, router_bias, T, E, d, in->expert_scores, st, stream);
         if (rc != RF_OK) return rc;
     }
     if (rf::moe_topk_launch(in->expert_scores, T, E, K, in->seq_experts_index, in->seq_experts_softmax,
@@ -318,46 +338,50 @@ int moe_layer(MoEInputRaw* in, bool compute_router, const float* router_bias, cu
                                in->permuted_experts, in->permuted_rows, in->first_token_offset, in->rev_permuted_rows,
                                in->expanded_seq_softmax, aux.sort_scratch, stream) != cudaSuccess)
         return RF_ERR_CUDA;
-    if (fill_expanded &&
-        rf::moe_gather_rows_launch(in->input_seq, static_cast<const int*>(in->permuted_rows), T, TK, d * 2,
-                                   in->expanded_seq_input, st->num_sms, stream) != cudaSuccess)
+    void* rows = fill_expanded ? in->expanded_seq_input : in->expanded_fc2_output;
+    if (rf::moe_gather_rows_launch(in->input_seq, static_cast<const int*>(in->permuted_rows), T, TK, d * 2, rows,
+                                   st->num_sms, stream) != cudaSuccess)
         return RF_ERR_CUDA;
     const int t_misc = tm.mark();
     tm.span(1, t_begin, t_misc, 0.0);
 
-    // ---- routed experts: fc1 (gate and up in one pass, SwiGLU in the epilogue), fc2
-    if (fill_expanded)
-        rc = grouped_gemm(rf::kMoeGemmSwiglu, in->expanded_seq_input, TK, in->expert_weight_gate, in->expert_weight_up,
-                          E, static_cast<const int*>(in->first_token_offset), f, d, nullptr, in->expanded_fc1_output,
-                          aux, st, stream);
-    else
-        rc = grouped_gemm(rf::kMoeGemmSwiglu, in->input_seq, TK, in->expert_weight_gate, in->expert_weight_up, E,
-                          static_cast<const int*>(in->first_token_offset), f, d, nullptr, in->expanded_fc1_output, aux,
-                          st, stream, nullptr, nullptr, static_cast<const int*>(in->permuted_rows), T);
+    // ---- experts: fc1 (gate and up in one pass, SwiGLU in the epilogue), fc2.  A shared expert as wide as the routed
+    // ones joins their launches as one more group: alone its 16 + 28 column blocks would occupy 22 % of the chip while
+    // a small batch streams its weights.  With stage times asked for it runs by itself, so that each of the reference's
+    // stages keeps a time of its own; the arithmetic is the same.
+    const bool merged = fs == f && !metrics;
+    const int* offsets = static_cast<const int*>(in->first_token_offset);
+    std::vector<const void*> wg(in->expert_weight_gate, in->expert_weight_gate + E),
+        wu(in->expert_weight_up, in->expert_weight_up + E), wd(in->expert_weight_down, in->expert_weight_down + E);
+    wg.push_back(in->shared_expert_weight_gate);
+    wu.push_back(in->shared_expert_weight_up);
+    wd.push_back(in->shared_expert_weight_down);
+    AltGroup s1{in->input_seq, T, in->shared_fc1_output}, s2{in->shared_fc1_output, T, in->shared_fc2_output};
+    if ((rc = build_tiles(offsets, E, merged ? T : 0, aux, stream)) != RF_OK) return rc;
+    rc = grouped_gemm(0, rows, TK, wg.data(), wu.data(), E, f, d, in->expanded_fc1_output, aux, st, stream,
+                      merged ? s1 : AltGroup{});
     if (rc != RF_OK) return rc;
     const int t_fc1 = tm.mark();
     tm.span(3, t_misc, t_fc1, 2.0 * TK * (double)f * d * 2);
-    rc = grouped_gemm(rf::kMoeGemmPlain, in->expanded_fc1_output, TK, in->expert_weight_down, nullptr, E,
-                      static_cast<const int*>(in->first_token_offset), d, f, nullptr, in->expanded_fc2_output, aux, st,
-                      stream);
+    rc = grouped_gemm(1, in->expanded_fc1_output, TK, wd.data(), nullptr, E, d, f, in->expanded_fc2_output, aux, st, stream,
+                      merged ? s2 : AltGroup{});
     if (rc != RF_OK) return rc;
     const int t_fc2 = tm.mark();
     tm.span(4, t_fc1, t_fc2, 2.0 * TK * (double)f * d);
 
-    // ---- shared expert over all tokens
-    const void* sg[1] = {in->shared_expert_weight_gate};
-    const void* su[1] = {in->shared_expert_weight_up};
-    const void* sd[1] = {in->shared_expert_weight_down};
-    rc = grouped_gemm(rf::kMoeGemmSwiglu, in->input_seq, T, sg, su, 1, aux.single_offsets, fs, d, nullptr,
-                      in->shared_fc1_output, aux, st, stream);
-    if (rc != RF_OK) return rc;
-    const int t_s1 = tm.mark();
-    tm.span(5, t_fc2, t_s1, 2.0 * T * (double)fs * d * 2);
-    rc = grouped_gemm(rf::kMoeGemmPlain, in->shared_fc1_output, T, sd, nullptr, 1, aux.single_offsets, d, fs, nullptr,
-                      in->shared_fc2_output, aux, st, stream);
-    if (rc != RF_OK) return rc;
-    const int t_s2 = tm.mark();
-    tm.span(6, t_s1, t_s2, 2.0 * T * (double)fs * d);
+    // ---- shared expert over all tokens, unless it ran above
+    int t_s2 = t_fc2;
+    if (!merged) {
+        if ((rc = build_tiles(nullptr, 0, T, aux, stream)) != RF_OK) return rc;
+        rc = grouped_gemm(0, nullptr, 0, &wg[E], &wu[E], 0, fs, d, nullptr, aux, st, stream, s1);
+        if (rc != RF_OK) return rc;
+        const int t_s1 = tm.mark();
+        tm.span(5, t_fc2, t_s1, 2.0 * T * (double)fs * d * 2);
+        rc = grouped_gemm(1, nullptr, 0, &wd[E], nullptr, 0, d, fs, nullptr, aux, st, stream, s2);
+        if (rc != RF_OK) return rc;
+        t_s2 = tm.mark();
+        tm.span(6, t_s1, t_s2, 2.0 * T * (double)fs * d);
+    }
 
     // ---- weighted combine + shared add
     if (rf::moe_combine_launch(in->expanded_fc2_output, in->shared_fc2_output,
@@ -371,11 +395,10 @@ int moe_layer(MoEInputRaw* in, bool compute_router, const float* router_bias, cu
     return RF_OK;
 }
 
-// Fused row gather (rf_moe_set_fused_gather, or RF_MOE_FUSED_GATHER=1 at first use): rf_moe_forward and
-// rf_run_from_python let the first expert GEMM gather the token rows and leave expanded_seq_input unwritten.
-// Off by default: measured on B200 (T = 8192, 32 experts, top-4, 20 layers back to back) the layer takes
-// 3.67 ms with it against 3.60 ms with the separate gather pass; the 0.94 GB of copy traffic it saves costs
-// less than the cp.async row gather adds to the GEMM's loader.
+// rf_moe_set_fused_gather, or RF_MOE_FUSED_GATHER=1 at first use: rf_moe_forward and rf_run_from_python leave
+// expanded_seq_input unwritten.  (Gathering inside the first expert GEMM's loader is slower than a pass of its own: with
+// 16-byte cp.async copies a layer of 8192 tokens, 32 experts takes 6.07 ms, with TMA row gathers 5.65, with the pass
+// 3.52.)
 int g_fused_gather = -1;
 bool fill_expanded_default() {
     if (g_fused_gather < 0) {
@@ -558,11 +581,13 @@ int rf_moe_grouped_gemm(const void* x, int n_rows, const void* const* w_ptrs_hos
         return RF_ERR_BAD_SHAPE;
     DeviceState* st = rf::device_state();
     if (!st) return RF_ERR_CUDA;
+    if (n_rows == 0) return RF_OK;
     Aux aux;
-    if (!carve_aux(&aux, n_rows, n_groups)) return RF_ERR_CUDA;
-    return grouped_gemm(w2_ptrs_host ? rf::kMoeGemmSwiglu : rf::kMoeGemmPlain, x, n_rows, w_ptrs_host, w2_ptrs_host,
-                        n_groups, group_offsets_dev, n_dim, k_dim, nullptr, out, aux, st,
-                        reinterpret_cast<cudaStream_t>(stream));
+    if (!carve_aux(&aux, n_rows, n_groups, 0)) return RF_ERR_CUDA;
+    cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+    const int rc = build_tiles(group_offsets_dev, n_groups, 0, aux, s);
+    if (rc != RF_OK) return rc;
+    return grouped_gemm(0, x, n_rows, w_ptrs_host, w2_ptrs_host, n_groups, n_dim, k_dim, out, aux, st, s);
 }
 
 int rf_moe_grouped_gemm_scatter(const void* x, int n_rows, const void* const* w_ptrs_host,
@@ -578,11 +603,14 @@ int rf_moe_grouped_gemm_scatter(const void* x, int n_rows, const void* const* w_
         if (!pp.p[i] || ((uintptr_t)pp.p[i] & 15)) return RF_ERR_NULL_POINTER;
     DeviceState* st = rf::device_state();
     if (!st) return RF_ERR_CUDA;
+    if (n_rows == 0) return RF_OK;
     Aux aux;
-    if (!carve_aux(&aux, n_rows, n_groups)) return RF_ERR_CUDA;
-    return grouped_gemm(rf::kMoeGemmPlain, x, n_rows, w_ptrs_host, nullptr, n_groups, group_offsets_dev, n_dim, k_dim,
-                        nullptr, const_cast<void*>(x), aux, st, reinterpret_cast<cudaStream_t>(stream), row_dest_dev,
-                        &pp);
+    if (!carve_aux(&aux, n_rows, n_groups, 0)) return RF_ERR_CUDA;
+    cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+    const int rc = build_tiles(group_offsets_dev, n_groups, 0, aux, s);
+    if (rc != RF_OK) return rc;
+    return grouped_gemm(0, x, n_rows, w_ptrs_host, nullptr, n_groups, n_dim, k_dim, nullptr, aux, st, s, {},
+                        RowScatter{row_dest_dev, &pp});
 }
 
 int rf_moe_router_gemm(const void* x, const void* router_weight, const float* router_bias, int n_tokens,
@@ -592,14 +620,9 @@ int rf_moe_router_gemm(const void* x, const void* router_weight, const float* ro
         return RF_ERR_BAD_SHAPE;
     DeviceState* st = rf::device_state();
     if (!st) return RF_ERR_CUDA;
-    Aux aux;
-    if (!carve_aux(&aux, n_tokens, 1)) return RF_ERR_CUDA;
-    cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-    int rc = set_single_offsets(aux, n_tokens, s);
-    if (rc != RF_OK) return rc;
-    const void* rw[1] = {router_weight};
-    return grouped_gemm(rf::kMoeGemmRouter, x, n_tokens, rw, nullptr, 1, aux.single_offsets, n_experts, d_hidden,
-                        router_bias, expert_scores, aux, st, s);
+    if (n_tokens == 0) return RF_OK;
+    return router_gemm(x, router_weight, router_bias, n_tokens, n_experts, d_hidden, expert_scores, st,
+                       reinterpret_cast<cudaStream_t>(stream));
 }
 
 int rf_moe_combine(const void* expanded_fc2_output, const void* shared_fc2_output, const void* rev_permuted_rows,

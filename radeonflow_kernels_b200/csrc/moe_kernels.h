@@ -19,8 +19,19 @@ cudaError_t moe_combine_launch(const void* y, const void* shared_out, const int*
                                int n_tokens, int top_k, int row_bytes, void* out, cudaStream_t stream);
 // dst[0] = a, dst[1] = b (a one-group offsets array written in stream order)
 cudaError_t moe_set_range_launch(int* dst, int a, int b, cudaStream_t stream);
-cudaError_t moe_tile_list_launch(const int* offsets, int n_groups, int* tile_group, int* tile_row0, int* tile_chunk,
-                                 int* tile_count, cudaStream_t stream);
+// Row ranges [offsets[g], offsets[g + 1]) -> list of row tiles for the grouped GEMM.  With alt_rows > 0 the list
+// starts with the tiles of one more group, number n_groups, of rows [0, alt_rows) of a matrix of its own (the
+// shared expert's).  At most alt_rows / kMoeTileRows + rows / kMoeTileRows + n_groups + 1 tiles.
+struct MoeTile {
+    int group;      // weight set
+    int row0;       // first row
+    int rows;       // valid rows, 1 .. kMoeTileRows
+    int chunk;      // (first tile of the tile's chunk << 8) | tiles in the chunk
+};
+// counters: [0] = number of tiles, [1 .. kMoeItemCounters] = 0, the item counters of as many grouped GEMMs.
+constexpr int kMoeItemCounters = 2;
+cudaError_t moe_tile_list_launch(const int* offsets, int n_groups, int alt_rows, MoeTile* tiles, int* counters,
+                                 cudaStream_t stream);
 
 // ---- expert-parallel exchange over peer memory (moe_ep.cu)
 struct PeerPtrs {
@@ -75,47 +86,59 @@ cudaError_t moe_ep_rendezvous_launch(const PeerPtrs& sync, const int* counts, in
                                      int rank, int world, int epoch, int* status, cudaStream_t stream);
 
 // ---- grouped fp16 GEMM (moe_gemm.cu)
-enum MoeGemmMode {
-    kMoeGemmPlain = 0,    // out[r, n] = fp16(X[r,:] . W_g[:, n]); W_g is [K, N] row-major (N contiguous)
-    kMoeGemmSwiglu = 1,   // out[r, n] = fp16(SiLU(fp16(X.Wa_g)) * fp16(X.Wb_g))
-    kMoeGemmRouter = 2,   // out[r, n] = fp16(X[r,:] . W[n,:] + bias[n]); W is [N, K] row-major (K contiguous)
+// plain:  out[r, n] = fp16(X[r,:] . W_g[:, n]); W_g is [K, N] row-major (N contiguous)
+// SwiGLU: out[r, n] = fp16(SiLU(fp16(X.Wa_g)) * fp16(X.Wb_g))
+
+// Rows of one tile of the grouped GEMM (the MMA's N), and the largest run of tiles of one group that the grouped
+// GEMM walks together (see tile_list_kernel).
+constexpr int kMoeTileRows = 256;
+constexpr int kMoeChunkTiles = 8;
+
+// Tensor maps of a fp16 row-major [rows, k] matrix whose rows are the GEMM's tokens: box[i] is 16 (i + 1) rows x 64
+// columns, so that half a tile of any height is one load.
+struct MoeRowMaps {
+    CUtensorMap box[kMoeTileRows / 32];
 };
 
-// Largest run of row tiles of one group that the grouped GEMM walks together (see tile_list_kernel).
-constexpr int kMoeChunkTiles = 16;
-
 struct MoeGemmParams {
-    const int* tile_group;      // [n_tiles] group (expert) of each 128-row tile
-    const int* tile_row0;       // [n_tiles] first row of the tile
-    const int* tile_chunk;      // [n_tiles] (first tile of the tile's chunk << 8) | tiles in the chunk
+    const MoeTile* tiles;       // row tiles (device)
     const int* tile_count;      // [1]
-    const int* group_offsets;   // [n_groups + 1] row range of each group
-    const CUtensorMap* b_maps;  // device array, one tensor map per group (first weight)
-    const CUtensorMap* b2_maps; // second weight per group (SwiGLU mode), else unused
-    const float* bias;          // router mode: optional fp32 [n_out]
+    int* next_item;             // [1] items drawn so far beyond each pair's first; 0 at the launch
+    const CUtensorMap* w_maps;  // device array, one tensor map per group (first weight)
+    const CUtensorMap* w2_maps; // second weight per group (SwiGLU mode), else unused
     void* out;                  // fp16 [rows, n_out]
+    // Group `alt_group` (-1: none) reads its rows from the `alt` maps and writes to alt_out: the shared expert, whose
+    // rows are the tokens themselves, runs in the same launch as the routed experts.
+    int alt_group;
+    void* alt_out;
     // Plain mode only, optional: row r of the result is stored to row (scatter_meta[r] & slot mask) of the
     // fp16 [*, n_out] matrix scatter_dst.p[scatter_meta[r] >> kEpMetaSlotBits] instead of out[r] (peer stores:
     // the expert outputs travel back to the GPUs that own the tokens from the GEMM's own epilogue).
     const int* scatter_meta;
     PeerPtrs scatter_dst;
-    // SwiGLU mode only, optional: row r of the A operand is row (gather_map[min(r, gather_rows - 1)] % gather_mod)
-    // of the fp16 [gather_mod, k] matrix gather_src (the token rows, read in place: the row gather of
-    // expand_input, src/moe/moe_topk_kernel.cpp:174-213, done by the GEMM's own loader); tma_a is then unused.
-    const void* gather_src;
-    const int* gather_map;
-    int gather_mod;
-    int gather_rows;
     int n_out;                  // output columns
     int k;                      // reduction length (multiple of 64)
-    int tma_store;              // 1: full 32-row slabs leave through the output tensor map
     int* status;                // device status area (status_words.h)
     int launch_tag;             // tag recorded with an expired wait
 };
 
-cudaError_t moe_gemm_launch(int mode, const CUtensorMap& tma_a, const CUtensorMap& tma_out, const MoeGemmParams& p,
+// x: the operand rows; alt: the alt group's rows.  `num_sms` = most CTAs to launch (two per cluster).
+cudaError_t moe_gemm_launch(bool swiglu, const MoeRowMaps& x, const MoeRowMaps& alt, const MoeGemmParams& p,
                             int num_sms, cudaStream_t stream);
-// Output columns covered by one tile in the given mode (256, or 128 for SwiGLU).
-int moe_gemm_tile_n(int mode);
+
+// ---- router GEMM (moe_router.cu)
+// out[r, n] = fp16(X[r,:] . W[n,:] + bias[n]); W is [N, K] row-major (K contiguous), N <= 256
+struct MoeRouterParams {
+    const float* bias;          // optional fp32 [n_out]
+    void* out;                  // fp16 [n_rows, n_out]
+    int n_rows;
+    int n_out;
+    int k;
+    int tma_store;              // 1: full 32-row slabs leave through the output tensor map
+    int* status;
+    int launch_tag;
+};
+cudaError_t moe_router_launch(const CUtensorMap& tma_x, const CUtensorMap& tma_w, const CUtensorMap& tma_out,
+                              const MoeRouterParams& p, int num_sms, cudaStream_t stream);
 
 }  // namespace rf

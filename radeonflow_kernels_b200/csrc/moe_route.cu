@@ -5,7 +5,7 @@
 //                        (src/moe/moe.cpp:119-126, src/moe/moe_topk_kernel.cpp:152-172, :199-201)
 //   gather_rows_kernel   expanded_seq_input[dest] = x[permuted_rows[dest] % T]  (:174-213)
 //   combine_kernel       out[t] = sum_i w * Y[rev[i*T+t]] + shared[t]           (:215-251)
-//   tile_list_kernel     per-expert row ranges -> list of 128-row tiles for the grouped GEMM
+//   tile_list_kernel     per-expert row ranges -> list of row tiles for the grouped GEMM
 #include "moe_kernels.h"
 
 #include <cuda_fp16.h>
@@ -287,23 +287,28 @@ combine_kernel(const uint4* __restrict__ y, const uint4* __restrict__ shared_out
     }
 }
 
-// Row ranges [offsets[g], offsets[g+1]) -> list of 128-row tiles: tile_group[i], tile_row0[i];
-// tile_count[0] = number of tiles.  One block; groups <= 1024.
-// tile_chunk[i] = (first tile of i's chunk << 8) | tiles in the chunk.  A chunk is a run of at most
-// kMoeChunkTiles consecutive tiles of ONE group (a group's tiles are split into equal chunks); the grouped
-// GEMM walks a chunk column block by column block, so the CTAs that run at the same time share one
-// group's weight column block and the chunk's row tiles.
+// Row ranges [offsets[g], offsets[g+1]) -> list of row tiles (and, first, the tiles of the alt group's alt_rows rows).
+// A group's rows are cut into the fewest tiles of at most kMoeTileRows rows, all of one height (a multiple of 16,
+// the step of the MMA's N) but the last: 1056 rows become four tiles of 224 and one of 160, not four of 256 and one
+// of 32 whose weight traffic would count in full.  One block; at most 1024 groups, the alt group included.
+// A chunk is a run of at most kMoeChunkTiles consecutive tiles of ONE group (a group's tiles are split into equal
+// chunks); the grouped GEMM walks a chunk column block by column block, so the pairs that run at the same time share
+// one group's weight column block and the chunk's row tiles.
 __global__ void __launch_bounds__(1024)
-tile_list_kernel(const int* __restrict__ offsets, int n_groups, int* __restrict__ tile_group,
-                 int* __restrict__ tile_row0, int* __restrict__ tile_chunk, int* __restrict__ tile_count) {
+tile_list_kernel(const int* __restrict__ offsets, int n_groups, int alt_rows, MoeTile* __restrict__ tiles,
+                 int* __restrict__ counters) {
     __shared__ int warp_sums[32];
-    const int g = threadIdx.x;
-    const int lane = g & 31, warp = g >> 5;
-    int lo = 0, n = 0;
-    if (g < n_groups) {
+    // with an alt group, thread 0 holds it and thread g + 1 group g
+    const int g = (int)threadIdx.x - (alt_rows > 0 ? 1 : 0);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int lo = 0, rows = 0;
+    if (g < 0) {
+        rows = alt_rows;
+    } else if (g < n_groups) {
         lo = offsets[g];
-        n = (offsets[g + 1] - lo + 127) >> 7;
+        rows = offsets[g + 1] - lo;
     }
+    const int n = (rows + kMoeTileRows - 1) / kMoeTileRows;
     int incl = n;
 #pragma unroll
     for (int s = 1; s < 32; s <<= 1) {
@@ -323,12 +328,11 @@ tile_list_kernel(const int* __restrict__ offsets, int n_groups, int* __restrict_
     }
     __syncthreads();
     const int start = (warp > 0 ? warp_sums[warp - 1] : 0) + incl - n;
+    const int height = n ? ((rows + n - 1) / n + 15) & ~15 : 0;
     const int n_chunks = (n + kMoeChunkTiles - 1) / kMoeChunkTiles;
     const int base = n_chunks ? n / n_chunks : 0;
     const int rem = n_chunks ? n % n_chunks : 0;          // the first `rem` chunks hold base + 1 tiles
     for (int i = 0; i < n; ++i) {
-        tile_group[start + i] = g;
-        tile_row0[start + i] = lo + i * 128;
         int c_first, c_size;
         if (i < rem * (base + 1)) {
             c_size = base + 1;
@@ -337,22 +341,14 @@ tile_list_kernel(const int* __restrict__ offsets, int n_groups, int* __restrict_
             c_size = base;
             c_first = rem * (base + 1) + ((i - rem * (base + 1)) / base) * base;
         }
-        tile_chunk[start + i] = ((start + c_first) << 8) | c_size;
+        tiles[start + i] = MoeTile{g < 0 ? n_groups : g, lo + i * height, min(height, rows - i * height),
+                                   ((start + c_first) << 8) | c_size};
     }
-    if (g == 1023) tile_count[0] = start + n;
-}
-
-__global__ void set_range_kernel(int* dst, int a, int b) {
-    dst[0] = a;
-    dst[1] = b;
+    if (threadIdx.x == 1023) counters[0] = start + n;
+    if (threadIdx.x < kMoeItemCounters) counters[1 + threadIdx.x] = 0;
 }
 
 }  // namespace
-
-cudaError_t moe_set_range_launch(int* dst, int a, int b, cudaStream_t stream) {
-    set_range_kernel<<<1, 1, 0, stream>>>(dst, a, b);
-    return cudaGetLastError();
-}
 
 cudaError_t moe_topk_launch(const void* scores, int n_tokens, int n_experts, int top_k, void* index, void* weight,
                             void* source_rows, cudaStream_t stream) {
@@ -415,9 +411,9 @@ cudaError_t moe_combine_launch(const void* y, const void* shared_out, const int*
     return cudaGetLastError();
 }
 
-cudaError_t moe_tile_list_launch(const int* offsets, int n_groups, int* tile_group, int* tile_row0, int* tile_chunk,
-                                 int* tile_count, cudaStream_t stream) {
-    tile_list_kernel<<<1, 1024, 0, stream>>>(offsets, n_groups, tile_group, tile_row0, tile_chunk, tile_count);
+cudaError_t moe_tile_list_launch(const int* offsets, int n_groups, int alt_rows, MoeTile* tiles, int* counters,
+                                 cudaStream_t stream) {
+    tile_list_kernel<<<1, 1024, 0, stream>>>(offsets, n_groups, alt_rows, tiles, counters);
     return cudaGetLastError();
 }
 

@@ -92,14 +92,30 @@ __device__ __forceinline__ unsigned long long wait_limit_ns(const int* status) {
         *reinterpret_cast<const volatile unsigned long long*>(status + kStatusLimitWord);
     return v ? v : kWaitTimeoutNs;
 }
+// CLUSTER: the wait also acquires what another CTA of the cluster released with its arrive.
+__device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+        "selp.u32 %0, 1, 0, p;\n"
+        "}\n"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int* status, int code, int tag) {
-    if (mbar_try_wait(bar, parity)) return true;
+    auto poll = [&] { return CLUSTER ? mbar_try_wait_cluster(bar, parity) : mbar_try_wait(bar, parity); };
+    if (poll()) return true;
     // The polling loop stays as small as possible (the waiting warps share their schedulers with the warps
     // that do the work); the clock is first read after 256 failed polls, so a wait that ends within a few
     // microseconds never touches it.
     unsigned long long t0 = 0;
     for (uint32_t it = 1;; ++it) {
-        if (mbar_try_wait(bar, parity)) return true;
+        if (poll()) return true;
         if ((it & 0xffu) == 0) {
             const int seen = *reinterpret_cast<volatile int*>(status);
             if (seen != 0 && (seen >> kStatusTagShift) == tag) return false;
@@ -151,17 +167,6 @@ __device__ __forceinline__ void griddep_launch_dependents() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-// ---------------------------------------------------------------- cp.async --
-// 16-byte asynchronous copy global -> shared (L2 only), for rows that a TMA box cannot address (gathered rows).
-__device__ __forceinline__ void cp_async_16(uint32_t dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-
 // --------------------------------------------------------------------- TMA --
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* m) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(m)) : "memory");
@@ -191,6 +196,15 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* m, 
         ::"r"(dst), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
         : "memory");
 }
+// The same load inside a CTA pair: `bar` (a shared::cluster address) may be a barrier of either CTA of the pair,
+// the destination is this CTA's own shared memory.
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* m, uint32_t bar, int c0, int c1) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 "
+        "[%0], [%1, {%3, %4}], [%2];"
+        ::"r"(dst), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar), "r"(c0), "r"(c1)
+        : "memory");
+}
 // 2-D tiled store shared -> global (bulk-group completion).
 __device__ __forceinline__ void tma_store_2d(const CUtensorMap* m, uint32_t src, int c0, int c1) {
     asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
@@ -201,6 +215,11 @@ __device__ __forceinline__ void tma_store_3d(const CUtensorMap* m, uint32_t src,
     asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];"
                  ::"l"(reinterpret_cast<uint64_t>(m)), "r"(src), "r"(c0), "r"(c1), "r"(c2)
                  : "memory");
+}
+__device__ __forceinline__ uint32_t ld_shared_u32(uint32_t addr) {
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+    return v;
 }
 __device__ __forceinline__ uint4 ld_shared_v4(uint32_t addr) {
     uint4 v;
@@ -288,6 +307,10 @@ __device__ __forceinline__ uint32_t mapa_cluster(uint32_t local_smem_addr, uint3
     uint32_t r;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local_smem_addr), "r"(rank));
     return r;
+}
+// 32-bit store into the shared memory of a CTA of the cluster.
+__device__ __forceinline__ void st_cluster_u32(uint32_t cluster_addr, uint32_t v) {
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cluster_addr), "r"(v) : "memory");
 }
 // Arrive on an mbarrier that may live in another CTA of the cluster.
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
@@ -439,6 +462,58 @@ __device__ __forceinline__ void reg_fence(float (&v)[32]) {
 __device__ __forceinline__ void tmem_ld_fence2(float (&v0)[32], float (&v1)[32]) {
     tmem_ld_fence(v0);
     reg_fence(v1);
+}
+
+// 16 lanes x 32 consecutive fp32 columns in the layout of four 16 x 8 mma accumulator fragments: thread i receives,
+// for fragment q, rows i/4 (v[4q], v[4q+1]) and i/4 + 8 (v[4q+2], v[4q+3]) at columns 8q + 2(i%4) + {0, 1}.
+// Asynchronous: valid after tmem_ld_wait16.
+__device__ __forceinline__ void tmem_ld_16x256b_x4_async(uint32_t taddr, float (&v)[16]) {
+    uint32_t* r = reinterpret_cast<uint32_t*>(v);
+    asm volatile(
+        "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr)
+        : "memory");
+}
+__device__ __forceinline__ void tmem_ld_wait16(float (&a)[16], float (&b)[16]) {
+    uint32_t* r = reinterpret_cast<uint32_t*>(a);
+    uint32_t* q = reinterpret_cast<uint32_t*>(b);
+    asm volatile(
+        "tcgen05.wait::ld.sync.aligned;\n"
+        : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+          "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]),
+          "+r"(q[0]), "+r"(q[1]), "+r"(q[2]), "+r"(q[3]), "+r"(q[4]), "+r"(q[5]), "+r"(q[6]), "+r"(q[7]),
+          "+r"(q[8]), "+r"(q[9]), "+r"(q[10]), "+r"(q[11]), "+r"(q[12]), "+r"(q[13]), "+r"(q[14]), "+r"(q[15])
+        :
+        : "memory");
+}
+// Four 8 x 8 matrices of 16-bit elements, each stored transposed: thread i holds elements (i/4, 2(i%4) + {0, 1}) of
+// every matrix and gives the 16-byte row address (i % 8) of matrix i / 8; row c of the stored matrix is column c.
+__device__ __forceinline__ void stmatrix_x4_trans(uint32_t addr, uint32_t m0, uint32_t m1, uint32_t m2, uint32_t m3) {
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};"
+                 ::"r"(addr), "r"(m0), "r"(m1), "r"(m2), "r"(m3)
+                 : "memory");
+}
+// Barrier `id` (1..15) among `n` threads of the CTA.
+__device__ __forceinline__ void named_barrier(int id, int n) {
+    asm volatile("barrier.sync %0, %1;" ::"r"(id), "r"(n) : "memory");
+}
+// The same with a vote: true in every thread iff `pred` is true in all of them.
+__device__ __forceinline__ bool named_barrier_all(int id, int n, bool pred) {
+    uint32_t r;
+    asm volatile(
+        "{\n"
+        ".reg .pred p, q;\n"
+        "setp.ne.b32 p, %3, 0;\n"
+        "barrier.red.and.pred q, %1, %2, p;\n"
+        "selp.u32 %0, 1, 0, q;\n"
+        "}\n"
+        : "=r"(r)
+        : "r"(id), "r"(n), "r"((uint32_t)pred)
+        : "memory");
+    return r != 0;
 }
 
 // Shared-memory matrix descriptor for a K-major operand tile stored as rows of

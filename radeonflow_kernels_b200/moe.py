@@ -104,8 +104,8 @@ def moe_forward(x, weights, config, expert_scores=None, router_bias=None, metric
     `expert_scores` given  -> `run_topk` (the reference entry: logits are an input; every stage tensor is written);
     `expert_scores` None   -> the router GEMM runs on the device (optional fp32 bias).  With `fill_stages` it is
     followed by `run_topk`, so that every stage tensor of the reference's checker is written; without, the
-    one-call entry `rf_moe_forward` runs (which, with `rf_moe_set_fused_gather(1)`, lets its first expert GEMM
-    gather the token rows itself and leaves `expanded_seq_input` unwritten).
+    one-call entry `rf_moe_forward` runs (which, with `rf_moe_set_fused_gather(1)`, leaves `expanded_seq_input`
+    unwritten).
     """
     L = _lib.lib()
     buf = MoEBuffers(x, weights, config, expert_scores)

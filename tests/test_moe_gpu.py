@@ -371,3 +371,65 @@ def test_grouped_gemm_scatter_equals_plain_grouped_gemm_then_permute(rf_lib):
                           if sizes[g]])
     ok, nbad, mx = o.check(plain.cpu().numpy(), ref)
     assert ok, (nbad, mx)
+
+
+@pytest.mark.parametrize("swiglu", [False, True])
+@pytest.mark.parametrize("k_dim,n_dim", [(64, 64), (64, 2048), (448, 320), (1024, 192)])
+def test_grouped_gemm_at_the_edges_of_its_tiles(rf_lib, k_dim, n_dim, swiglu):
+    """Group sizes around the tile height (256), its 16-row step and the 32-row epilogue step; column counts that end
+    inside a column block; K of one step (every pair then draws more items than it has slots for).  Against fp32
+    products: a product is one fp16 rounding away (2^-11), plus what another order of the fp32 sums can flip (one more
+    step of 2^-10); behind SiLU(g) * u the steps of g and u arrive scaled by the other factor and |SiLU'| <= 1.1."""
+    sizes = [1, 0, 15, 16, 17, 31, 33, 127, 128, 129, 240, 255, 256, 257, 0, 512, 513, 2049, 4100]
+    offsets = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int32)
+    rows = int(offsets[-1])
+    g = torch.Generator(device=DEV).manual_seed(k_dim + n_dim)
+    x = torch.randn(rows, k_dim, generator=g, device=DEV).half()
+
+    def weights():
+        return [(torch.randn(k_dim, n_dim, generator=g, device=DEV) / k_dim ** 0.5).half() for _ in sizes]
+
+    w, w2 = weights(), weights() if swiglu else None
+    doff = torch.from_numpy(offsets).to(DEV)
+
+    def table(ws):
+        return (ctypes.c_void_p * len(ws))(*[t.data_ptr() for t in ws]) if ws else None
+
+    canary = 0x7BFF
+    out = torch.full((rows + 8, n_dim), canary, dtype=torch.int16, device=DEV).view(torch.float16)
+    assert rf_lib.rf_moe_grouped_gemm(x.data_ptr(), rows, table(w), table(w2), doff.data_ptr(), len(sizes), n_dim,
+                                      k_dim, out.data_ptr(), None) == 0
+    torch.cuda.synchronize()
+    assert G.device_status() == 0
+    assert (out[rows:].view(torch.int16) == canary).all()
+    for i, (lo, hi) in enumerate(zip(offsets[:-1], offsets[1:])):
+        if lo == hi:
+            continue
+        p1 = x[lo:hi].double() @ w[i].double()
+        if swiglu:
+            gate, up = p1.half().double(), (x[lo:hi].double() @ w2[i].double()).half().double()
+            silu = torch.nn.functional.silu(gate)
+            ref = silu.half().double() * up
+            bound = 2.0 ** -10 * (1.1 * gate.abs() * up.abs() + 2.0 * ref.abs() + silu.abs() * up.abs()) + 2.0 ** -14
+        else:
+            ref, bound = p1, 1.5 * 2.0 ** -10 * p1.abs() + 2.0 ** -14
+        assert ((out[lo:hi].double() - ref).abs() <= bound).all(), (i, sizes[i])
+
+
+@pytest.mark.parametrize("d,f,e,k,t", [(512, 256, 8, 2, 1), (512, 256, 8, 2, 257), (192, 64, 4, 4, 130), (1024, 512, 32, 4, 1000)])
+@pytest.mark.parametrize("fused", [0, 1])
+def test_shared_expert_in_the_routed_launches_equals_launches_of_its_own(rf_lib, d, f, e, k, t, fused):
+    """Stage times asked for: the shared expert runs by itself; otherwise as one more group of the routed experts'
+    GEMMs.  Same bits either way, with the expert rows in expanded_seq_input and in expanded_fc2_output."""
+    x, w, cfg = o.generate_input(d, f, e, 1, k, t, 31)
+    tx, tw = torch.from_numpy(x).to(DEV), to_dev(w)
+    rf_lib.rf_moe_set_fused_gather(fused)
+    try:
+        _, a = M.moe_forward(tx, tw, cfg, fill_stages=False)
+        _, b = M.moe_forward(tx, tw, cfg, metrics=_lib.PerfMetrics(), fill_stages=False)
+    finally:
+        rf_lib.rf_moe_set_fused_gather(0)
+    torch.cuda.synchronize()
+    assert G.device_status() == 0
+    for name in ("expanded_fc1_output", "expanded_fc2_output", "shared_fc1_output", "shared_fc2_output", "final_output"):
+        assert torch.equal(a.stages[name], b.stages[name]), name
