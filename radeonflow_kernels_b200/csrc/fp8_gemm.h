@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
 #include <stddef.h>
+#include <stdint.h>
 
 namespace rf {
 
@@ -24,9 +25,9 @@ struct GemmParams {
     // (Measured on B200: with 16 more bytes of kernel parameters the short kernels ran 0.3-0.4 us slower per
     // launch, so the struct stays at 128 bytes.  The two members of the union are never used by one launch.)
     union {
-        const int* fnuz_flags;          // nullptr, or two device words left by the e4m3fnuz conversion pass
-                                        // (reference-layout entry only): [0] / [1] != 0 = read A / B from the
-                                        // converted copy (dests.m[0] / m[1])
+        const uint32_t* fnuz_words;     // nullptr, or the kFnuzWords device words left by the e4m3fnuz conversion
+                                        // pass (reference-layout entry only): bit 0 / 1 of their OR = read A / B
+                                        // from the converted copy (dests.m[0] / m[1])
         unsigned long long sk_token;    // stream-K: the value of a raised flag in this launch
     };
     int dest_first;         // first destination to store to (N-split: own rank, so ranks target different GPUs)
@@ -35,7 +36,7 @@ struct GemmParams {
     // fp32 slot per CTA, followed by one 64-bit flag per CTA; a flag is raised when it holds sk_token and is
     // cleared by the CTA that consumes it, so stale contents never pass for a raised flag.
     int sk_tiles;
-    GemmParams() : fnuz_flags(nullptr), sk_tiles(0) {}
+    GemmParams() : fnuz_words(nullptr), sk_tiles(0) {}
 };
 static_assert(sizeof(GemmParams) == 128, "kernel parameter block of the GEMM");
 
@@ -85,11 +86,16 @@ cudaError_t fp8_gemm_launch(const CUtensorMap& tma_a, const CUtensorMap& tma_b, 
 // `max_pieces` are written.
 int fp8_gemm_walk_pieces(const GemmParams& p, int unit, int n_units, int* out, int max_pieces);
 
-// One pass over `n_bytes` (multiple of 16) of e4m3fnuz data: writes the e4m3fn bytes of equal value to `dst`
-// and sets *flag (device word, cleared first) when the operand holds a byte that cannot be consumed as it
-// is (0x80, 0x7F, 0xFF); in that case kDiagFnuzByte is also OR-ed into the diagnostics word of `status`.
-cudaError_t fp8_fnuz_convert_launch(const void* src, void* dst, size_t n_bytes, int* flag, int* status, int num_sms,
-                                    cudaStream_t stream);
+// One pass over two operands of e4m3fnuz data (bytes: multiples of 16): writes the e4m3fn bytes of equal value to
+// a_dst / b_dst and kFnuzWords words (16-byte aligned), whose OR has bit 0 / 1 set when A / B holds a byte that cannot be
+// consumed as it is (0x80, 0x7F, 0xFF); in that case kDiagFnuzByte is also OR-ed into the diagnostics word of `status`.
+constexpr int kFnuzWords = 512;      // blocks of the pass, one word each
+cudaError_t fp8_fnuz_convert_launch(const void* a, void* a_dst, size_t a_bytes, const void* b, void* b_dst,
+                                    size_t b_bytes, uint32_t* words, int* status, cudaStream_t stream);
+
+// Whether a split-K launch of `tiles` 128 x 128 tiles in `splits` K slices runs inside clusters on the current device
+// (one launch, no scratch; false without a device).
+bool fp8_gemm_cluster_split(int tiles, int splits);
 
 // Sets the launch attributes of every GEMM kernel configuration on the current device (normally done
 // lazily by the first launch of each configuration).

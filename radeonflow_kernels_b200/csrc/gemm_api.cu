@@ -251,18 +251,18 @@ int gemm_impl(const void* a, const void* b, const float* as, const float* bs, vo
     rf::GemmDestMaps dests;
     bool use_dests = false;
     if (fnuz) {
-        // e4m3fnuz operands: one pass per operand writes the equal-valued e4m3fn bytes into library-owned
+        // e4m3fnuz operands: one pass over both writes the equal-valued e4m3fn bytes into library-owned
         // scratch and flags operands that hold +-240 or NaN bytes; the kernel reads a flagged operand from
         // its converted copy (maps in dests.m[0] / m[1]) and an unflagged one, exactly, from the caller's bytes.
         const size_t a_bytes = (size_t)m * k, b_bytes = (size_t)n * k;
         if (a_bytes % 16 != 0 || b_bytes % 16 != 0) return RF_ERR_BAD_SHAPE;
         const size_t a_pad = (a_bytes + 255) / 256 * 256, b_pad = (b_bytes + 255) / 256 * 256;
-        char* conv = static_cast<char*>(rf::device_scratch(a_pad + b_pad + 256, rf::kScratchFnuz));
+        char* conv = static_cast<char*>(
+            rf::device_scratch(a_pad + b_pad + rf::kFnuzWords * sizeof(uint32_t), rf::kScratchFnuz));
         if (!conv) return RF_ERR_CUDA;
-        int* flags = reinterpret_cast<int*>(conv + a_pad + b_pad);
-        if (rf::fp8_fnuz_convert_launch(a, conv, a_bytes, flags, st->status, st->num_sms, stream) != cudaSuccess ||
-            rf::fp8_fnuz_convert_launch(b, conv + a_pad, b_bytes, flags + 1, st->status, st->num_sms, stream) !=
-                cudaSuccess)
+        uint32_t* words = reinterpret_cast<uint32_t*>(conv + a_pad + b_pad);
+        if (rf::fp8_fnuz_convert_launch(a, conv, a_bytes, b, conv + a_pad, b_bytes, words, st->status, stream) !=
+            cudaSuccess)
             return RF_ERR_CUDA;
         if (!rf::encode_tma_2d(&dests.m[0], CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, conv, (uint64_t)k, (uint64_t)m,
                                (uint64_t)m, 128, 128, true) ||
@@ -270,7 +270,7 @@ int gemm_impl(const void* a, const void* b, const float* as, const float* bs, vo
                                (uint64_t)n, 128, 128, true))
             return RF_ERR_CUDA;
         for (int i = 2; i < 8; ++i) dests.m[i] = dests.m[0];
-        p.fnuz_flags = flags;
+        p.fnuz_words = words;
         use_dests = true;
     }
     if (n_dest > 1) {
