@@ -723,7 +723,7 @@ def run_gpu_arm(args):
     for s in shapes:
         sp = L.rf_fp8_gemm_choose_split(s["m"], s["n"], s["k"])
         s["split"] = sp
-        launches_per_step += 1 + (1 if sp > 1 else 0)
+        launches_per_step += L.rf_fp8_gemm_kernel_launches(s["m"], s["n"], s["k"])
 
     for _ in range(max(3, args.warmup)):
         sweep()

@@ -88,6 +88,10 @@ size_t rf_fp8_gemm_workspace_bytes(int m, int n, int k, int split_k);
  * RF_SPLIT_STREAMK when it would run the shape as a stream-K pass.            */
 int rf_fp8_gemm_choose_split(int m, int n, int k);
 
+/* Kernels that one row-major GEMM of this shape launches under the library's own plan: 1, or 2 where split-K slices
+ * go through memory and a fix-up kernel sums them (0 for a bad shape or without a device).                        */
+int rf_fp8_gemm_kernel_launches(int m, int n, int k);
+
 /* Introspection, no GPU needed: the work CTA `cta` of a launch on `num_sms` SMs goes through, in order, as
  * computed on the host by the code the kernel itself runs.  Four ints per piece: tile number, K slice, first
  * K block, end K block.  block_n 128 or 256; split_k >= 1 or RF_SPLIT_STREAMK.  Returns the number of pieces

@@ -101,6 +101,8 @@ def _declare(L: ctypes.CDLL) -> None:
     L.rf_fp8_gemm.argtypes = [vp, vp, vp, vp, vp, ci, ci, ci, ci, vp, sz, vp]
     L.rf_fp8_gemm_workspace_bytes.restype = sz
     L.rf_fp8_gemm_workspace_bytes.argtypes = [ci, ci, ci, ci]
+    L.rf_fp8_gemm_kernel_launches.restype = ci
+    L.rf_fp8_gemm_kernel_launches.argtypes = [ci, ci, ci]
     L.rf_fp8_gemm_choose_split.restype = ci
     L.rf_fp8_gemm_choose_split.argtypes = [ci, ci, ci]
     L.rf_fp8_gemm_set_plan.restype = ci

@@ -69,7 +69,7 @@ inline int gemm_streamk_tiles(int tiles, int num_sms) {
     return tiles < num_sms ? tiles : rem + num_sms;
 }
 
-// Launches the GEMM (and the split-K fix-up when p.splits > 1) on `stream`.
+// Launches the GEMM (and the split-K fix-up when p.splits > 1 and the slices do not meet in clusters) on `stream`.
 // `block_n` is the configuration the tensor map of B and p.tiles_m / p.tiles_n were built for.
 // `tma_c` stores bf16 C boxes of 32 rows x 64 columns; `tma_p` (used when p.splits > 1) stores fp32
 // slice boxes of 32 rows x 32 columns into the [splits][m][n] scratch.

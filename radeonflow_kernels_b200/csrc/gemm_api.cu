@@ -69,17 +69,19 @@ int streamk_region(int m, int n, int k, int bn, int num_sms) {
     return sk;
 }
 
-// Cost model, in units of one 128-deep K block of a 128 x 128 tile at full tensor rate
-// (about 0.14 us): rounds of tiles over the SMs x (K blocks per slice + fixed per-tile cost),
-// plus, for split-K, the fp32 slice round trip through HBM and the second launch.
+// Cost model, in units of one 128-deep K block of a 128 x 128 tile (about 0.27 us where one round of tiles fits the
+// chip: 64 x 576 x 7168 takes 17.7, 12.8, 8.9, 7.4 us with 56, 28, 14, 7 K blocks per CTA): rounds of tiles over the
+// SMs x (K blocks per slice + fixed per-tile cost), plus, for split-K, either the cluster's exchange (2.6 us in those
+// figures) or the fp32 slice round trip and the second launch (4.7 us in 512 x 1536 x 7168 with 3 slices).
 GemmPlan plan_for(int m, int n, int k, int num_sms, int bn, int forced_split) {
     const int tr = rf::gemm_tile_rows(bn), tc = rf::gemm_tile_cols(bn);
     const int tiles = ((m + tr - 1) / tr) * ((n + tc - 1) / tc);
     const int kb = k / kBlockK;
     if (rf::gemm_is_pair(bn)) num_sms /= 2;     // work items go to CTA pairs
     // relative time of one K block of one work item, from in-kernel cycle counts
-    // (128 x 128: ~620 cycles, 128 x 256: ~790, CTA pair 256 x 256: ~925)
-    const double tile_w = bn == 512 ? 1.5 : (bn == 256 ? 1.25 : (bn == 384 ? 0.8 : 1.0));
+    // (128 x 128: ~620 cycles, 128 x 256: ~790, CTA pair 256 x 256: ~925); with at most one item per SM, where latency
+    // and not the shared pipes decide, a 128 x 256 tile takes 0.42 us a K block
+    const double wide = bn == 512 ? 1.5 : (bn == 256 ? 1.25 : (bn == 384 ? 0.8 : 1.0));
     GemmPlan best{bn, 1, 1e30};
     for (int s = 1; s <= 8; ++s) {
         if (forced_split > 0 && s != forced_split) continue;
@@ -87,10 +89,13 @@ GemmPlan plan_for(int m, int n, int k, int num_sms, int bn, int forced_split) {
         if (s > kb) break;
         const int rounds = (tiles * s + num_sms - 1) / num_sms;
         const int kb_per = (kb + s - 1) / s;
+        const double tile_w = bn == 256 && rounds == 1 ? 1.5 : wide;
         double cost = (double)rounds * (kb_per * tile_w + 4.0);
-        if (s > 1) {
+        if (s > 1 && bn == 128 && rf::fp8_gemm_cluster_split(tiles, s)) {
+            cost += 10.0;
+        } else if (s > 1) {
             const double bytes = 8.0 * s * (double)m * n + 2.0 * (double)m * n;
-            cost += (bytes / 6.0e12 + 2.5e-6) / 0.14e-6;
+            cost += (bytes / 12.0e12 + 2.5e-6) / 0.27e-6;      // (slices of one round stay in L2)
         }
         if (cost < best.cost) best = GemmPlan{bn, s, cost};
     }
@@ -345,6 +350,16 @@ int rf_fp8_gemm_choose_split(int m, int n, int k) {
     rf::DeviceState* st = rf::device_state();
     if (!st) return 0;
     return choose_plan(m, n, k, st->num_sms, 0).splits;
+}
+
+int rf_fp8_gemm_kernel_launches(int m, int n, int k) {
+    if (!shape_ok(m, n, k)) return 0;
+    rf::DeviceState* st = rf::device_state();
+    if (!st) return 0;
+    const GemmPlan plan = choose_plan(m, n, k, st->num_sms, 0);
+    const int tiles = ((m + 127) / 128) * ((n + 127) / 128);
+    const bool fix_up = plan.splits > 1 && !(plan.block_n == 128 && rf::fp8_gemm_cluster_split(tiles, plan.splits));
+    return fix_up ? 2 : 1;
 }
 
 int rf_fp8_gemm_work_pieces(int m, int n, int k, int block_n, int split_k, int num_sms, int cta, int* pieces,

@@ -519,3 +519,36 @@ def test_fnuz_entry_against_reference_fixtures(rf_lib, path):
     torch.cuda.synchronize()
     assert G.device_status() == 0 and canary_intact(full, m, n)
     assert_close(c.view(torch.uint16).cpu().numpy(), z["c_bits"])
+
+
+@pytest.mark.parametrize("m,n", [(1, 64), (16, 192), (127, 128), (129, 320), (272, 576)])
+@pytest.mark.parametrize("split", [2, 3, 5, 8])
+def test_split_k_in_clusters_equals_split_k_through_memory(rf_lib, m, n, split):
+    """128-wide tiles sum their K slices inside a cluster, 256-wide ones through memory and a fix-up kernel: the same
+    slices in the same order, so the same bits; ragged rows and columns, slices of unequal length."""
+    k = 128 * (2 * split + 1)
+    a, b, a_s, b_s = o.generate_input(m, n, k, 77)
+    got = {}
+    for block_n in (128, 256):
+        assert rf_lib.rf_fp8_gemm_set_plan(m, n, k, block_n, split) == 0
+        assert rf_lib.rf_fp8_gemm_kernel_launches(m, n, k) == (1 if block_n == 128 else 2)
+        got[block_n] = run_gemm(a, b, a_s, b_s)
+        if m % 16 == 0:
+            got[block_n, "mn"] = run_mn_major(rf_lib, a, b, a_s, b_s)
+    assert rf_lib.rf_fp8_gemm_set_plan(m, n, k, 0, 0) == 0
+    assert np.array_equal(got[128], got[256])
+    if m % 16 == 0:
+        assert np.array_equal(got[128, "mn"], got[128]) and np.array_equal(got[256, "mn"], got[128])
+    assert_close(got[128], o.fp8_gemm(a, b, a_s, b_s))
+
+
+def run_mn_major(rf_lib, a, b, a_s, b_s):
+    """The same operands through the reference-layout entry."""
+    m, n = a.shape[0], b.shape[0]
+    full, c = canary_output(m, n)
+    at, bt, ast, bst = gemm_device_inputs(*(np.ascontiguousarray(t.T) for t in (a, b, a_s, b_s)))
+    assert rf_lib.rf_fp8_gemm_colmajor(at.data_ptr(), bt.data_ptr(), ast.data_ptr(), bst.data_ptr(), c.data_ptr(), m, n,
+                                       a.shape[1], None, 0, None) == 0
+    torch.cuda.synchronize()
+    assert G.device_status() == 0 and canary_intact(full, m, n)
+    return c.view(torch.uint16).cpu().numpy()
