@@ -274,7 +274,7 @@ int router_gemm(const void* x, const void* w, const float* bias, int n_rows, int
         !rf::encode_tma_2d(&tx, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, x, (uint64_t)n_rows, (uint64_t)k, (uint64_t)k * 2,
                            128, 64, true) ||
         !rf::encode_tma_2d(&tw, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, w, (uint64_t)n_out, (uint64_t)k, (uint64_t)k * 2,
-                           256, 64, true))
+                           (uint32_t)(n_out + 15) / 16 * 16, 64, true))
         return RF_ERR_CUDA;
     rf::MoeRouterParams p;
     p.tma_store = n_out % 64 == 0;

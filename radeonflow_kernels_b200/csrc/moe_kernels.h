@@ -126,7 +126,7 @@ struct MoeGemmParams {
 cudaError_t moe_gemm_launch(bool swiglu, const MoeRowMaps& x, const MoeRowMaps& alt, const MoeGemmParams& p,
                             int num_sms, cudaStream_t stream);
 
-// ---- router GEMM (moe_router.cu)
+// ---- router GEMM (moe_router.cu); tma_w: boxes of n_out rounded up to 16 rows x 64 columns
 // out[r, n] = fp16(X[r,:] . W[n,:] + bias[n]); W is [N, K] row-major (K contiguous), N <= 256
 struct MoeRouterParams {
     const float* bias;          // optional fp32 [n_out]

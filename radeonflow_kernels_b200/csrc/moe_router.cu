@@ -1,9 +1,14 @@
 // Router GEMM of the MoE layer on sm_100a: logits[t, e] = fp16(X[t,:] . W[e,:] + bias[e]).
 //
 // Replaces the PyTorch router matmul (scripts/gen_submission.py:400).  One CTA per 128-row tile, warp-specialised:
-//   warp 0     TMA producer: A tile [128 x 64] fp16 and one box of 256 weight rows x 64, both K-major, 128-byte swizzle
-//   warp 1     MMA issuer: 4 x tcgen05.mma.kind::f16 (128 x 256 x 16) per stage, whole K accumulated in TMEM
+//   warp 0     TMA producer: A tile [128 x 64] fp16 and one box of the weight's rows x 64, both K-major, 128-byte swizzle
+//   warp 1     MMA issuer: 4 x tcgen05.mma.kind::f16 (128 x N x 16) per stage, whole K accumulated in TMEM
 //   warps 4-11 epilogue of the previous tile while the next tile's MMAs run
+//
+// What bounds it: one tile's K loop, whose loads come from HBM, so the time is K steps x latency / stages in flight.  N is
+// the experts rounded up to 16, and the stages are as small as that allows and as many as fit: 32 experts take 9 stages of
+// 20 KB where boxes of 256 rows took 4 of 48.  128 tokens, K = 7168: 42.1 -> 32.0 us, 8192 tokens 49.0 -> 36.8.  (K is
+// not split over CTAs: sums in another order round single logits the other way, and a token then chooses another expert.)
 #include "ptx.cuh"
 #include "moe_kernels.h"
 
@@ -12,34 +17,33 @@ namespace rf {
 namespace {
 
 constexpr int BM = 128;
-constexpr int BN = 256;          // MMA N, TMEM columns per accumulator buffer
+constexpr int BN = 256;          // largest MMA N, TMEM columns per accumulator buffer
 constexpr int BK = 64;           // 128 bytes of fp16: one swizzle row
 constexpr int UMMA_K = 16;
-constexpr int STAGES = 4;
-constexpr int A_BYTES = BM * BK * 2;        // 16 KB
-constexpr int B_BYTES = BN * BK * 2;        // 32 KB
-constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
+constexpr int MAX_STAGES = 9;
+constexpr int RING_BYTES = 192 * 1024;
+constexpr int A_BYTES = BM * BK * 2;        // 16 KB; B: 128 bytes for each of the MMA's N rows
 constexpr int NUM_NON_EPI_WARPS = 4;
 constexpr int EPI_WARPS = 8;
 constexpr int THREADS = 32 * (NUM_NON_EPI_WARPS + EPI_WARPS);
 constexpr int SLAB_BYTES = 32 * 128;
 constexpr int NBUF = 2;
 constexpr int TMEM_COLS = NBUF * BN;
-constexpr int BAR_BYTES = (2 * STAGES + 2 * NBUF) * 8 + 16;
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + EPI_WARPS * SLAB_BYTES + BAR_BYTES + 1024;
+constexpr int BAR_BYTES = (2 * MAX_STAGES + 2 * NBUF) * 8 + 16;
+constexpr int SMEM_BYTES = RING_BYTES + EPI_WARPS * SLAB_BYTES + BAR_BYTES + 1024;
 
 __global__ void __launch_bounds__(THREADS, 1)
 moe_router_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                   const __grid_constant__ CUtensorMap tma_out, const MoeRouterParams p) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    const uint32_t slab_base = smem_base + STAGES * STAGE_BYTES;
+    const uint32_t slab_base = smem_base + RING_BYTES;
     const uint32_t bar_base = slab_base + EPI_WARPS * SLAB_BYTES;
     auto full_bar = [&](int s) { return bar_base + 8u * s; };
-    auto empty_bar = [&](int s) { return bar_base + 8u * (STAGES + s); };
-    auto tmem_full_bar = [&](int b) { return bar_base + 8u * (2 * STAGES + b); };
-    auto tmem_empty_bar = [&](int b) { return bar_base + 8u * (2 * STAGES + NBUF + b); };
-    const uint32_t tmem_slot = bar_base + 8u * (2 * STAGES + 2 * NBUF);
+    auto empty_bar = [&](int s) { return bar_base + 8u * (MAX_STAGES + s); };
+    auto tmem_full_bar = [&](int b) { return bar_base + 8u * (2 * MAX_STAGES + b); };
+    auto tmem_empty_bar = [&](int b) { return bar_base + 8u * (2 * MAX_STAGES + NBUF + b); };
+    const uint32_t tmem_slot = bar_base + 8u * (2 * MAX_STAGES + 2 * NBUF);
     uint32_t* tmem_slot_ptr = reinterpret_cast<uint32_t*>(smem_raw + (tmem_slot - smem_u32(smem_raw)));
 
     const int warp = threadIdx.x >> 5;
@@ -47,7 +51,7 @@ moe_router_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
 
     if (threadIdx.x == 0) {
         tma_prefetch_desc(&tma_a);
-        for (int s = 0; s < STAGES; ++s) {
+        for (int s = 0; s < MAX_STAGES; ++s) {
             mbar_init(full_bar(s), 1);
             mbar_init(empty_bar(s), 1);
         }
@@ -68,31 +72,33 @@ moe_router_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
 
     const int total_work = (p.n_rows + BM - 1) / BM;
     const int k_steps = p.k / BK;
+    const int n_mma = (p.n_out + 15) & ~15;
+    const uint32_t stage_bytes = A_BYTES + n_mma * (BK * 2);
+    const uint32_t n_stages = min((uint32_t)MAX_STAGES, RING_BYTES / stage_bytes);
 
     if (warp == 0) {
         // ------------------------------------------------------ TMA producer
-        uint32_t it = 0;
+        uint32_t s = 0, ph = 0;       // stage, parity of its use
         bool ok = true;
         for (int w = blockIdx.x; w < total_work && ok; w += gridDim.x) {
             const int row0 = w * BM;
-            for (int ks = 0; ks < k_steps; ++ks, ++it) {
-                const int s = it % STAGES;
-                const uint32_t ph = (it / STAGES) & 1;
+            for (int ks = 0; ks < k_steps; ++ks) {
                 ok = __all_sync(0xffffffffu, mbar_wait(empty_bar(s), ph ^ 1, p.status, kErrProducerWait, p.launch_tag));
                 if (!ok) break;
                 if (elect_one()) {
-                    mbar_expect_tx(full_bar(s), STAGE_BYTES);
-                    const uint32_t sa = smem_base + s * STAGE_BYTES;
+                    mbar_expect_tx(full_bar(s), stage_bytes);
+                    const uint32_t sa = smem_base + s * stage_bytes;
                     tma_load_2d(sa, &tma_a, full_bar(s), ks * BK, row0);
                     tma_load_2d(sa + A_BYTES, &tma_b, full_bar(s), ks * BK, 0);
                 }
                 __syncwarp();
+                if (++s == n_stages) { s = 0; ph ^= 1; }
             }
         }
     } else if (warp == 1) {
         // -------------------------------------------------------- MMA issuer
-        constexpr uint32_t idesc = make_idesc(BM, BN, /*f16*/ 0, /*f16*/ 0, 0, 0);
-        uint32_t it = 0, tcount = 0;
+        const uint32_t idesc = make_idesc(BM, n_mma, /*f16*/ 0, /*f16*/ 0, 0, 0);
+        uint32_t s = 0, ph = 0, tcount = 0;
         bool ok = true;
         for (int w = blockIdx.x; w < total_work && ok; w += gridDim.x, ++tcount) {
             const int buf = tcount & 1;
@@ -100,13 +106,11 @@ moe_router_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
             ok = __all_sync(0xffffffffu, mbar_wait(tmem_empty_bar(buf), bph ^ 1, p.status, kErrMmaWaitTmem, p.launch_tag));
             if (!ok) break;
             const uint32_t d = tmem_base + buf * BN;
-            for (int ks = 0; ks < k_steps; ++ks, ++it) {
-                const int s = it % STAGES;
-                const uint32_t ph = (it / STAGES) & 1;
+            for (int ks = 0; ks < k_steps; ++ks) {
                 ok = __all_sync(0xffffffffu, mbar_wait(full_bar(s), ph, p.status, kErrMmaWaitFull, p.launch_tag));
                 if (!ok) break;
                 tc_fence_after();
-                const uint32_t sa = smem_base + s * STAGE_BYTES;
+                const uint32_t sa = smem_base + s * stage_bytes;
                 const uint64_t adesc = smem_desc_kmajor_sw128(sa);
                 const uint64_t bdesc = smem_desc_kmajor_sw128(sa + A_BYTES);
                 if (elect_one()) {
@@ -118,6 +122,7 @@ moe_router_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
                     if (ks == k_steps - 1) umma_commit(tmem_full_bar(buf));
                 }
                 __syncwarp();
+                if (++s == n_stages) { s = 0; ph ^= 1; }
             }
         }
     } else if (warp >= NUM_NON_EPI_WARPS) {
