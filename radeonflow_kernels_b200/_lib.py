@@ -6,8 +6,6 @@ resolved, importing the binding raises.
 import ctypes
 import os
 
-import torch
-
 PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(PKG_DIR, "librf_b200.so")
 
@@ -64,14 +62,21 @@ class MoEInputRaw(ctypes.Structure):
 
 _lib = None
 
-# The raw handle of the current stream of the current device.  torch.cuda.current_stream() builds a Stream object
-# first: 3.4 us per call against 0.2 us, which a GEMM of 6 us waits for (1024 x 4096 x 512 through custom_kernel:
-# 12.6 us of host time with it).
-_get_device = torch._C._cuda_getDevice
-_get_raw_stream = torch._C._cuda_getCurrentRawStream
+_get_device = _get_raw_stream = None
 
 
 def current_stream() -> int:
+    """The raw handle of the current stream of the current device.
+
+    torch.cuda.current_stream() builds a Stream object first: 3.4 us per call against 0.2 us, which a GEMM of 6 us
+    waits for (1024 x 4096 x 512 through custom_kernel: 12.6 us of host time with it).  Bound at the first call: the
+    binding itself needs neither torch nor a torch with CUDA.
+    """
+    global _get_device, _get_raw_stream
+    if _get_raw_stream is None:
+        import torch
+        _get_device = torch._C._cuda_getDevice
+        _get_raw_stream = torch._C._cuda_getCurrentRawStream
     return _get_raw_stream(_get_device())
 
 

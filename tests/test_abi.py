@@ -3,6 +3,10 @@ and rejects bad arguments before touching the GPU."""
 import ctypes
 import os
 import re
+import subprocess
+import sys
+
+import pytest
 
 from radeonflow_kernels_b200 import _lib
 
@@ -120,3 +124,17 @@ def test_missing_library_fails_loudly(monkeypatch, tmp_path):
     monkeypatch.setattr(_lib, "LIB_PATH", str(tmp_path / "nope.so"))
     with pytest.raises(RuntimeError, match="no CPU or PyTorch fallback"):
         _lib.lib()
+
+
+@pytest.mark.parametrize("without", [
+    # no torch at all: the binding as a file of its own
+    "sys.modules['torch'] = None; import importlib.util as u; s = u.spec_from_file_location('b', {path!r});"
+    " m = u.module_from_spec(s); s.loader.exec_module(m); assert b'sm_100a' in m.lib().rf_version()",
+    # a torch built without CUDA: the package
+    "import torch; [delattr(torch._C, n) for n in ('_cuda_getDevice', '_cuda_getCurrentRawStream')"
+    " if hasattr(torch._C, n)]; import radeonflow_kernels_b200 as p; assert p._lib.lib()",
+], ids=["torch", "torch with CUDA"])
+def test_binding_loads_without(rf_lib, without):
+    code = "import sys; " + without.format(path=_lib.__file__)
+    res = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True)
+    assert res.returncode == 0, res.stderr
