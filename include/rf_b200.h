@@ -106,7 +106,7 @@ int rf_fp8_gemm_work_pieces(int m, int n, int k, int block_n, int split_k, int n
  * The library starts with a built-in table for the benchmark shapes (RF_FP8_GEMM_NO_BUILTIN_PLANS=1 drops
  * it) and reads the file named by RF_FP8_GEMM_PLANS at first use.                                       */
 int rf_fp8_gemm_set_plan(int m, int n, int k, int block_n, int split_k);
-/* The plan the library would use (table entry or cost model; 148 SMs assumed when no GPU is present).   */
+/* The plan the library would use (table entry or cost model; without a GPU that of a B200 with 148 SMs).  */
 int rf_fp8_gemm_get_plan(int m, int n, int k, int *block_n, int *split_k);
 /* Text file, one "m n k block_n split_k" per line, '#' comments (what `python -m
  * radeonflow_kernels_b200.tune` writes).  Returns the number of entries loaded, -1 if the file cannot be

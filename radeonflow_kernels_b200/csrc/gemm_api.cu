@@ -69,6 +69,14 @@ int streamk_region(int m, int n, int k, int bn, int num_sms) {
     return sk;
 }
 
+// Whether the planner reckons with the K slices of `tiles` 128 x 128 tiles meeting in clusters: clusters of 2 .. 8 CTAs
+// that a B200 holds at once, as it answers itself.  A table and not a question to the device, so that a plan is the same
+// with and without one; whether a launch really runs in clusters is asked of its device (fp8_gemm_cluster_split).
+bool plan_in_clusters(int tiles, int splits) {
+    constexpr int kClusters[9] = {0, 0, 74, 45, 33, 26, 22, 15, 15};
+    return splits >= 2 && splits <= 8 && tiles <= kClusters[splits];
+}
+
 // Cost model, in units of one 128-deep K block of a 128 x 128 tile (about 0.27 us where one round of tiles fits the
 // chip: 64 x 576 x 7168 takes 17.7, 12.8, 8.9, 7.4 us with 56, 28, 14, 7 K blocks per CTA): rounds of tiles over the
 // SMs x (K blocks per slice + fixed per-tile cost), plus, for split-K, either the cluster's exchange (2.6 us in those
@@ -91,7 +99,7 @@ GemmPlan plan_for(int m, int n, int k, int num_sms, int bn, int forced_split) {
         const int kb_per = (kb + s - 1) / s;
         const double tile_w = bn == 256 && rounds == 1 ? 1.5 : wide;
         double cost = (double)rounds * (kb_per * tile_w + 4.0);
-        if (s > 1 && bn == 128 && rf::fp8_gemm_cluster_split(tiles, s)) {
+        if (s > 1 && bn == 128 && plan_in_clusters(tiles, s)) {
             cost += 10.0;
         } else if (s > 1) {
             const double bytes = 8.0 * s * (double)m * n + 2.0 * (double)m * n;

@@ -1,11 +1,16 @@
 """Tuned-plan table of the FP8 GEMM (the replacement of the reference's dispatch table and tuner,
 src/gemm/gemm_launcher.cpp:229-247, tuner/gemm_tuner.py): host logic on CPU, effect on the GPU."""
 import ctypes
+import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
 
 from radeonflow_kernels_b200 import tune
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
 def _get(L, m, n, k):
@@ -35,6 +40,29 @@ def test_builtin_table_covers_the_benchmark_shapes(rf_lib):
     for (m, n, k) in tune.BENCHMARK_SHAPES:
         bn, s = _get(rf_lib, m, n, k)
         assert bn in (128, 256, 512) and (1 <= s <= k // 128 or s == tune.STREAM_K)
+
+
+def _plan_list():
+    """Plans of shapes around the lines between one pass, split-K in clusters and split-K through memory."""
+    from radeonflow_kernels_b200 import _lib
+    return [_get(_lib.lib(), m, n, k) for m in (1, 64, 200, 1025, 3000) for n in (64, 576, 1536, 4160)
+            for k in (1024, 2176, 4864, 7168)]
+
+
+def test_plan_without_a_device(rf_lib):
+    """The plan of a B200 where there is none: slices of 128-wide tiles whose clusters fit that chip meet in them."""
+    assert _get(rf_lib, 64, 576, 7168) == (128, 8)
+    assert _get(rf_lib, 200, 1536, 7168) == (128, 5)
+    assert _get(rf_lib, 200, 4160, 4864) == (128, 2)
+
+
+@pytest.mark.gpu
+def test_plan_is_the_same_with_and_without_a_device(rf_lib):
+    code = "from tests.test_gemm_plans import _plan_list; print(_plan_list())"
+    res = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True,
+                         env=dict(os.environ, CUDA_VISIBLE_DEVICES=""))
+    assert res.returncode == 0, res.stderr
+    assert res.stdout.strip().splitlines()[-1] == str(_plan_list())
 
 
 def test_load_plans_file(rf_lib, tmp_path):
