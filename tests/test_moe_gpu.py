@@ -373,14 +373,20 @@ def test_grouped_gemm_scatter_equals_plain_grouped_gemm_then_permute(rf_lib):
     assert ok, (nbad, mx)
 
 
+@pytest.mark.parametrize("ctas", [0, 4])
 @pytest.mark.parametrize("swiglu", [False, True])
 @pytest.mark.parametrize("k_dim,n_dim", [(64, 64), (64, 2048), (448, 320), (1024, 192)])
-def test_grouped_gemm_at_the_edges_of_its_tiles(rf_lib, k_dim, n_dim, swiglu):
+def test_grouped_gemm_at_the_edges_of_its_tiles(rf_lib, k_dim, n_dim, swiglu, ctas):
     """Group sizes around the tile height (256), its 16-row step and the 32-row epilogue step; column counts that end
-    inside a column block; K of one step (every pair then draws more items than it has slots for).  Against fp32
-    products: a product is one fp16 rounding away (2^-11), plus what another order of the fp32 sums can flip (one more
-    step of 2^-10); behind SiLU(g) * u the steps of g and u arrive scaled by the other factor and |SiLU'| <= 1.1."""
+    inside a column block; K of one step, where the producer runs furthest ahead.  On the whole chip a pair draws a few
+    items; two pairs (grid limit 4) draw so many that the 16 slots in which drawn items are announced are used again,
+    with either parity.  Against fp32 products: a product is one fp16 rounding away (2^-11), plus what another order of
+    the fp32 sums can flip (one more step of 2^-10); behind SiLU(g) * u the steps of g and u arrive scaled by the other
+    factor and |SiLU'| <= 1.1."""
     sizes = [1, 0, 15, 16, 17, 31, 33, 127, 128, 129, 240, 255, 256, 257, 0, 512, 513, 2049, 4100]
+    if ctas:
+        items = sum(-(-n // 256) for n in sizes) * -(-n_dim // (128 if swiglu else 256))
+        assert items // (ctas // 2) > (2 * 16 if n_dim == 2048 else 16)
     offsets = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int32)
     rows = int(offsets[-1])
     g = torch.Generator(device=DEV).manual_seed(k_dim + n_dim)
@@ -397,8 +403,13 @@ def test_grouped_gemm_at_the_edges_of_its_tiles(rf_lib, k_dim, n_dim, swiglu):
 
     canary = 0x7BFF
     out = torch.full((rows + 8, n_dim), canary, dtype=torch.int16, device=DEV).view(torch.float16)
-    assert rf_lib.rf_moe_grouped_gemm(x.data_ptr(), rows, table(w), table(w2), doff.data_ptr(), len(sizes), n_dim,
-                                      k_dim, out.data_ptr(), None) == 0
+    assert rf_lib.rf_moe_set_grid_limit(ctas) == 0
+    try:
+        st = rf_lib.rf_moe_grouped_gemm(x.data_ptr(), rows, table(w), table(w2), doff.data_ptr(), len(sizes), n_dim,
+                                        k_dim, out.data_ptr(), None)
+    finally:
+        rf_lib.rf_moe_set_grid_limit(0)
+    assert st == 0
     torch.cuda.synchronize()
     assert G.device_status() == 0
     assert (out[rows:].view(torch.int16) == canary).all()
