@@ -502,6 +502,51 @@ def test_fnuz_nan_byte_stays_nan(rf_lib):
     assert G.device_status() == 16 and G.device_status() == 0
 
 
+@pytest.mark.parametrize("where", ["nowhere", "a end", "b end", "a middle, b third quarter", "everywhere"])
+def test_fnuz_conversion_over_several_strides(rf_lib, where):
+    """The conversion pass takes 2 MiB of (A, B) per stride of its grid and four strides per iteration: operands of
+    16.03 MiB, A ending inside the second stride, a third iteration of which hardly anything is left.  Special bytes in
+    the last 16 bytes of A or of B, in strides between, or all over.  Bit for bit the e4m3fn entry's result on bytes
+    converted here: a flagged operand at equal value, an unflagged one as it is with its scales halved."""
+    m, n, k = 1040, 7168, 2048
+    rng = np.random.default_rng(9)
+
+    def operand(rows):
+        x = rng.integers(0, 256, size=(k, rows), dtype=np.uint8)
+        x[np.isin(x, (0x80, 0x7F, 0xFF))] = 0x38
+        return x, rng.uniform(0.5, 2.0, size=(k // 128, -(-rows // (1 if rows == m else 128)))).astype(np.float32)
+
+    (a, a_s), (b, b_s) = operand(m), operand(n)
+    flat_a, flat_b = a.reshape(-1), b.reshape(-1)
+    if where == "everywhere":
+        flat_a[::97], flat_b[5::101] = 0x7F, 0xFF
+    elif where != "nowhere":
+        if where.startswith("a"):
+            flat_a[-3 if where == "a end" else flat_a.size // 2] = 0xFF
+        if "b" in where:
+            flat_b[-1 if where == "b end" else flat_b.size * 3 // 4] = 0x7F
+    byte = np.arange(256)
+    mag, sign = byte & 0x7F, byte & 0x80
+    lut = (sign | np.where(mag >= 16, mag - 8, (mag + ((mag >> 1) & 1)) >> 1)).astype(np.uint8)
+
+    def as_e4m3fn(x, sc):
+        flagged = ((x & 0x7F) == 0x7F).any()
+        return (lut[x], sc) if flagged else (x, sc * np.float32(0.5))
+
+    from tests.helpers import to_dev
+    got = []
+    for entry, ops in ((rf_lib.rf_fp8_gemm_colmajor_fnuz, (a, b, a_s, b_s)),
+                       (rf_lib.rf_fp8_gemm_colmajor, [t for pair in zip(as_e4m3fn(a, a_s), as_e4m3fn(b, b_s)) for t in pair])):
+        dev = [to_dev(t) for t in ops]
+        full, c = canary_output(m, n)
+        assert entry(*[t.data_ptr() for t in dev], c.data_ptr(), m, n, k, None, 0, None) == 0
+        torch.cuda.synchronize()
+        assert canary_intact(full, m, n)
+        assert G.device_status() == (16 if entry is rf_lib.rf_fp8_gemm_colmajor_fnuz and where != "nowhere" else 0)
+        got.append(c.view(torch.uint16).cpu().numpy())
+    assert np.array_equal(got[0], got[1])
+
+
 @pytest.mark.parametrize("path", GOLDEN_FNUZ, ids=[os.path.basename(p) for p in GOLDEN_FNUZ])
 def test_fnuz_entry_against_reference_fixtures(rf_lib, path):
     """The reference's own data path (e4m3fnuz bytes, [k][m] / [k][n] storage) through `rf_fp8_gemm_colmajor_fnuz`
