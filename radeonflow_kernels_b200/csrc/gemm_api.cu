@@ -69,18 +69,23 @@ int streamk_region(int m, int n, int k, int bn, int num_sms) {
     return sk;
 }
 
-// Whether the planner reckons with the K slices of `tiles` 128 x 128 tiles meeting in clusters: clusters of 2 .. 8 CTAs
-// that a B200 holds at once, as it answers itself.  A table and not a question to the device, so that a plan is the same
-// with and without one; whether a launch really runs in clusters is asked of its device (fp8_gemm_cluster_split).
+// Whether the planner reckons with the K slices of `tiles` 128 x 128 tiles meeting in clusters: fewer clusters of 2 .. 8
+// CTAs than a B200 answers that it holds at once (with all 45 clusters of 3 in use 50 x 5696 x 2304 takes 9.5 us, one
+// pass 7.7).  A table and not a question to the device, so that a plan is the same with and without one; whether a
+// launch runs in clusters is asked of its device (fp8_gemm_cluster_split).
 bool plan_in_clusters(int tiles, int splits) {
     constexpr int kClusters[9] = {0, 0, 74, 45, 33, 26, 22, 15, 15};
-    return splits >= 2 && splits <= 8 && tiles <= kClusters[splits];
+    return splits >= 2 && splits <= 8 && tiles < kClusters[splits];
 }
 
 // Cost model, in units of one 128-deep K block of a 128 x 128 tile (about 0.27 us where one round of tiles fits the
 // chip: 64 x 576 x 7168 takes 17.7, 12.8, 8.9, 7.4 us with 56, 28, 14, 7 K blocks per CTA): rounds of tiles over the
-// SMs x (K blocks per slice + fixed per-tile cost), plus, for split-K, either the cluster's exchange (2.6 us in those
-// figures) or the fp32 slice round trip and the second launch (4.7 us in 512 x 1536 x 7168 with 3 slices).
+// SMs x (K blocks per slice + fixed per-tile cost), plus, for split-K, either the cluster's exchange (3.0 us) or the fp32
+// slices and the second launch (3.2 us; with less than one 32-row box of rows 5.7; behind the longer epilogue of a
+// 256-wide tile 4.9).  The constants are those that lose least over 2009 shapes of up to 300 tiles, each timed under every
+// plan in a CUDA graph: 1.2 % on the geometric mean against the fastest plan.  (With 2.5 us for every second launch it was
+// 3.3 %: 4 x 6080 x 2176 was split in 3 slices, 9.7 us where a plain pass takes 7.6, and 50 x 4480 x 4864 in 8 wide
+// ones, 11.7 us where 4 of 128 take 9.4.)
 GemmPlan plan_for(int m, int n, int k, int num_sms, int bn, int forced_split) {
     const int tr = rf::gemm_tile_rows(bn), tc = rf::gemm_tile_cols(bn);
     const int tiles = ((m + tr - 1) / tr) * ((n + tc - 1) / tc);
@@ -88,8 +93,12 @@ GemmPlan plan_for(int m, int n, int k, int num_sms, int bn, int forced_split) {
     if (rf::gemm_is_pair(bn)) num_sms /= 2;     // work items go to CTA pairs
     // relative time of one K block of one work item, from in-kernel cycle counts
     // (128 x 128: ~620 cycles, 128 x 256: ~790, CTA pair 256 x 256: ~925); with at most one item per SM, where latency
-    // and not the shared pipes decide, a 128 x 256 tile takes 0.42 us a K block
+    // and not the shared pipes decide, a 128 x 256 tile takes 0.38 us a K block
     const double wide = bn == 512 ? 1.5 : (bn == 256 ? 1.25 : (bn == 384 ? 0.8 : 1.0));
+    // One 128 x 128 tile per SM, its K loop no longer than the host takes for two launches (about 9.4 us).  Called in a
+    // loop, one pass against 3 slices through memory: 50 x 5888 x 2560 8.4 / 9.5 us, 64 x 5888 x 3072 9.3 / 9.4, 64 x
+    // 5888 x 3712 10.6 / 9.4.
+    const bool short_pass = kb + 4 <= 28 && ((m + 127) / 128) * ((n + 127) / 128) <= num_sms;
     GemmPlan best{bn, 1, 1e30};
     for (int s = 1; s <= 8; ++s) {
         if (forced_split > 0 && s != forced_split) continue;
@@ -97,13 +106,14 @@ GemmPlan plan_for(int m, int n, int k, int num_sms, int bn, int forced_split) {
         if (s > kb) break;
         const int rounds = (tiles * s + num_sms - 1) / num_sms;
         const int kb_per = (kb + s - 1) / s;
-        const double tile_w = bn == 256 && rounds == 1 ? 1.5 : wide;
+        const double tile_w = bn == 256 && rounds == 1 ? 1.4 : wide;
         double cost = (double)rounds * (kb_per * tile_w + 4.0);
         if (s > 1 && bn == 128 && plan_in_clusters(tiles, s)) {
-            cost += 10.0;
+            cost += 11.0;
         } else if (s > 1) {
-            const double bytes = 8.0 * s * (double)m * n + 2.0 * (double)m * n;
-            cost += (bytes / 12.0e12 + 2.5e-6) / 0.27e-6;      // (slices of one round stay in L2)
+            if (short_pass && forced_split <= 0) continue;
+            const double bytes = 8.0 * s * (double)m * n + 2.0 * (double)m * n;      // (slices of one round stay in L2)
+            cost += bytes / 16.0e12 / 0.27e-6 + (bn == 128 ? (m < 32 ? 21.0 : 12.0) : 18.0);
         }
         if (cost < best.cost) best = GemmPlan{bn, s, cost};
     }
@@ -128,16 +138,19 @@ GemmPlan choose_plan_inner(int m, int n, int k, int num_sms, int forced_split) {
     }
     // Stream-K instead of a plain single pass, in K blocks of the chosen tile: a plain pass takes
     // rounds x (kb + per-tile cost), a stream-K pass the even share of all K blocks plus its fixed cost (slot
-    // write, slot read, one more piece per CTA: 7-11 us measured on B200, about 18 K blocks of a 128 x 256 tile).
-    // That pays when a long-K shape has just over a whole number of waves (160 tiles of 56 K blocks: 2 x 56
-    // against 60.5 + 18); none of the 18 benchmark shapes is such a shape.
+    // write, slot read, one more piece per CTA).  Behind whole waves that is about 18 K blocks of a 128 x 256 tile
+    // (7-11 us measured on B200), which pays when a long-K shape has just over a whole number of waves (160 tiles of
+    // 56 K blocks: 2 x 56 against 60.5 + 18); none of the 18 benchmark shapes is such a shape.  With fewer tiles than
+    // SMs every tile has several contributors and a K block takes half the time: about 50 K blocks (256 wide 90;
+    // medians of 154 shapes; 300 x 4160 x 7168 takes 26.6 us, a plain pass 18.1).
     if (forced_split == 0 && best.splits == 1 && !rf::gemm_is_pair(best.block_n) &&
         streamk_region(m, n, k, best.block_n, num_sms) > 0) {
         const int kb = k / kBlockK;
         const int tiles = ((m + 127) / 128) * ((n + best.block_n - 1) / best.block_n);
         const int rounds = (tiles + num_sms - 1) / num_sms;
         const double plain = (double)rounds * (kb + 3.0);
-        const double shared = (double)tiles * kb / num_sms + 3.0 * (tiles / num_sms + 1) + 18.0;
+        const double fixed = rounds > 1 ? 18.0 : (best.block_n == 256 ? 90.0 : 50.0);
+        const double shared = (double)tiles * kb / num_sms + 3.0 * (tiles / num_sms + 1) + fixed;
         if (shared < plain) best.splits = kStreamK;
     }
     return best;

@@ -56,6 +56,23 @@ def test_plan_without_a_device(rf_lib):
     assert _get(rf_lib, 200, 4160, 4864) == (128, 2)
 
 
+@pytest.mark.parametrize("m,n,k,plan", [
+    # a few rows, a wide output: the second launch costs more than it saves (us, this plan / split through memory)
+    (4, 6080, 2176, (128, 1)),       # 7.6 / 9.7 in 3 slices
+    (3, 5760, 2048, (128, 1)),       # 7.6 / 9.6 in 4 wide slices
+    (50, 6784, 2560, (128, 1)),      # 8.3 / 10.7 in 5 wide slices
+    # 128-wide slices beat wide ones of the same rounds
+    (50, 4480, 4864, (128, 4)),      # 9.4 / 11.7 in 8 wide slices
+    (50, 3904, 6784, (128, 4)),      # 9.9 / 11.9 in 8 wide slices
+    # but a split through memory pays where it halves a long K loop, and more slices than two in clusters
+    (6000, 64, 4096, (128, 3)),      # 8.9 / 10.3 in 2 slices in clusters
+    # stream-K does not pay with fewer tiles than SMs
+    (300, 4160, 7168, (128, 1)),     # 18.1 / stream-K 26.6
+])
+def test_plan_of_shapes_where_the_costs_are_close(rf_lib, m, n, k, plan):
+    assert _get(rf_lib, m, n, k) == plan
+
+
 @pytest.mark.gpu
 def test_plan_is_the_same_with_and_without_a_device(rf_lib):
     code = "from tests.test_gemm_plans import _plan_list; print(_plan_list())"
