@@ -38,7 +38,7 @@ def _check_fp16_cuda(name, t):
         raise ValueError(f"moe: {name} must be a contiguous CUDA fp16 tensor (there is no CPU path)")
 
 
-@functools.lru_cache(maxsize=None)
+@functools.lru_cache(maxsize=48)       # three per expert count
 def _expert_names(n_experts, j):
     return tuple(f"experts.{i}.{j}.weight" for i in range(n_experts))
 
@@ -49,6 +49,8 @@ def _expert_ptrs(weights, n_experts, j, ctype):
     A layer of 32 experts has 96 of these tensors and nothing is enqueued before their addresses are known, so the
     loop does no more than it must: names made once per expert count, one condition per tensor.
     """
+    if n_experts > 0:
+        weights[f"experts.{n_experts - 1}.{j}.weight"]      # KeyError before names are made that no weight has
     ts = [weights[name] for name in _expert_names(n_experts, j)]
     f16 = torch.float16
     for t in ts:

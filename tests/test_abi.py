@@ -138,3 +138,14 @@ def test_binding_loads_without(rf_lib, without):
     code = "import sys; " + without.format(path=_lib.__file__)
     res = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True)
     assert res.returncode == 0, res.stderr
+
+
+def test_an_expert_count_beyond_the_weights_is_refused_without_work(rf_lib):
+    """The names of a layer's experts are kept from call to call: a bounded number of layers' worth, and none for a
+    configuration whose weights are not there."""
+    from radeonflow_kernels_b200 import moe
+    known = moe._expert_names.cache_info()
+    with pytest.raises(KeyError):
+        moe._expert_ptrs({"experts.0.0.weight": None}, 100_000, 0, ctypes.c_void_p)
+    assert moe._expert_names.cache_info().misses == known.misses
+    assert known.maxsize is not None
