@@ -50,8 +50,11 @@ SWEEP = [(m, n, k) for m in (1024, 6144) for (n, k) in NK_PAIRS]
 # Reads = A + B + scales once; C mostly stays in the 126 MB L2 at kernel end, hence traffic < algorithmic.
 NCU_DRAM_BYTES = [18649344, 6402816, 11740928, 2173440, 16908032, 40669696, 19015680, 11283712, 2697984, 57371392,
                   14570240, 49792255, 30637824, 61002752, 116749312, 66869760, 49148928, 5439488]
-# same two counters for the largest moe_gemm_kernel launch of the single-GPU MoE layer (routed fc1)
-MOE_NCU_DRAM_BYTES = 2.91e9
+# same two counters for the largest moe_gemm_kernel launch of the single-GPU MoE layer (fc1 of the routed experts and the
+# shared one)
+MOE_NCU_DRAM_BYTES = 2.99e9
+# kernels of one layer through rf_moe_forward: router, top-k, sort (3), row gather, tile list, fc1, fc2, combine
+MOE_LAYER_LAUNCHES = 10
 METRIC = "fp8_blockscaled_gemm_tflops"
 UNIT = "TFLOP/s"
 
@@ -480,8 +483,8 @@ def run_extras(args, rank, world, dev, dist, peaks):
                      "frac": fl / (ms * 1e-3) / 1e12 / f16_peak,
                      "frac_of_sustained_peak": fl / (ms * 1e-3) / 1e12 / peaks["bf16_tflops_sustained"],
                      "kernel": "moe_gemm_kernel", "traffic": MOE_NCU_DRAM_BYTES,
-                     "traffic_note": "DRAM bytes of the largest moe_gemm_kernel launch of the layer (routed fc1), ncu; "
-                                     "algorithmic 2.48e9; achieved is layer FLOPs over layer time (all kernels)",
+                     "traffic_note": "DRAM bytes of the largest moe_gemm_kernel launch of the layer (fc1), ncu; "
+                                     "algorithmic 2.69e9; achieved is layer FLOPs over layer time (all kernels)",
                      "peak_source": f"bf16_tflops of {peaks['source']} (the layer runs for milliseconds at the power "
                                     "cap: the sustained figure is the fairer one)"}}
     del buf, w, x
@@ -635,11 +638,11 @@ def run_moe_only(args):
         "roofline": {"bound": "tensor", "achieved": fl / (ms * 1e-3) / 1e12, "peak": peaks["bf16_tflops"],
                      "unit": "TFLOP/s", "frac": fl / (ms * 1e-3) / 1e12 / peaks["bf16_tflops"],
                      "traffic": MOE_NCU_DRAM_BYTES,
-                     "traffic_note": "DRAM bytes of the largest moe_gemm_kernel launch (routed fc1), ncu capture; "
-                                     "algorithmic 2.48e9; achieved/frac are layer FLOPs over layer time (all "
+                     "traffic_note": "DRAM bytes of the largest moe_gemm_kernel launch (fc1), ncu capture; "
+                                     "algorithmic 2.69e9; achieved/frac are layer FLOPs over layer time (all "
                                      "kernels of the layer)",
                      "kernel": "moe_gemm_kernel"},
-        "gpu_launches": 18 * steps}), flush=True)
+        "gpu_launches": MOE_LAYER_LAUNCHES * steps}), flush=True)
 
 
 def run_multi_gpu_only(args):

@@ -444,3 +444,23 @@ def test_shared_expert_in_the_routed_launches_equals_launches_of_its_own(rf_lib,
     assert G.device_status() == 0
     for name in ("expanded_fc1_output", "expanded_fc2_output", "shared_fc1_output", "shared_fc2_output", "final_output"):
         assert torch.equal(a.stages[name], b.stages[name]), name
+
+
+def test_kernels_of_a_layer_are_as_many_as_the_benchmark_claims(rf_lib):
+    """`gpu_launches` of the layer's benchmark line is a count of kernels per layer: here they are counted."""
+    import bench
+    from torch.profiler import ProfilerActivity, profile
+    x, w, cfg = o.generate_input(512, 256, 8, 1, 2, 300, 3)
+    tx, tw = torch.from_numpy(x).to(DEV), to_dev(w)
+    buf = M.MoEBuffers(tx, tw, cfg)
+
+    def layer():
+        assert rf_lib.rf_moe_forward(ctypes.byref(buf.raw), None, None, None) == 0
+
+    layer()
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        layer()
+        torch.cuda.synchronize()
+    names = [e.name for e in prof.events() if e.device_type == torch.autograd.DeviceType.CUDA]
+    assert len(names) == bench.MOE_LAYER_LAUNCHES, names
