@@ -79,7 +79,9 @@ void run(void *a, void *b, void *as, void *bs, void *c, int m, int n, int k, Per
 int rf_fp8_gemm(const void *a, const void *b, const float *as, const float *bs, void *c, int m, int n, int k,
                 int split_k, void *workspace, size_t workspace_bytes, rf_stream_t stream);
 
-/* Scratch bytes rf_fp8_gemm needs for this shape and split (0 = library choice).
+/* Scratch bytes rf_fp8_gemm asks for at this shape and split (0 = library choice).  A plan with K slices asks for them
+ * also where its slices meet in clusters and leave them unused (rf_fp8_gemm_kernel_launches): one answer with and without
+ * a device, whatever clusters the device then holds.
  * Reference: init_workspace, src/gemm/gemm_launcher.cpp:30-36 (fixed 1.4 GB). */
 size_t rf_fp8_gemm_workspace_bytes(int m, int n, int k, int split_k);
 
@@ -351,7 +353,8 @@ int rf_moe_set_map_cache_sets(int max_sets);
 int rf_moe_set_fused_gather(int on);
 
 /* Grid cap of the grouped GEMMs that THIS host thread enqueues from now on (0 = one persistent CTA per SM,
- * the default).  The expert-parallel layer uses it to leave SMs to its dispatch kernel while the shared
+ * the default).  They run on pairs of CTAs: an odd cap is rounded down, and one pair is the least.  The router GEMM
+ * takes the cap as it is.  The expert-parallel layer uses it to leave SMs to its dispatch kernel while the shared
  * expert runs.  No reference counterpart.                                                             */
 int rf_moe_set_grid_limit(int max_ctas);
 

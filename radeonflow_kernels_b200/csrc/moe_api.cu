@@ -1,6 +1,6 @@
 // C-ABI entry points of the MoE layer (declared in include/rf_b200.h): stage sequencing, workspace
 // carving, per-expert tensor-map cache, per-stage timing.  Host code only; kernels live in
-// moe_route.cu and moe_gemm.cu.
+// moe_route.cu, moe_router.cu and moe_gemm.cu.
 #include "../../include/rf_b200.h"
 #include "host_util.h"
 #include "moe_kernels.h"
@@ -227,8 +227,9 @@ int build_tiles(const int* offsets_dev, int n_groups, int alt_rows, const Aux& a
                ? RF_OK : RF_ERR_CUDA;
 }
 
-// The `nth` grouped GEMM (< kMoeItemCounters) over the row tiles built last in `aux`: rows of `x` [n_rows, k] by per-group weights (w2_host: SwiGLU of the
-// two products).  With alt.rows > 0 the weight lists hold one entry more, the alt group's, behind the n_groups others.
+// The `nth` grouped GEMM (< kMoeItemCounters) over the row tiles built last in `aux`: rows of `x` [n_rows, k] by
+// per-group weights (w2_host: SwiGLU of the two products).  With alt.rows > 0 the weight lists hold one entry more, the
+// alt group's, behind the n_groups others.
 int grouped_gemm(int nth, const void* x, int n_rows, const void* const* w_host, const void* const* w2_host, int n_groups,
                  int n_out, int k, void* out, const Aux& aux, DeviceState* st, cudaStream_t stream,
                  const AltGroup& alt = {}, const RowScatter& scatter = {}) {
@@ -346,8 +347,8 @@ int moe_layer(MoEInputRaw* in, bool compute_router, const float* router_bias, cu
     tm.span(1, t_begin, t_misc, 0.0);
 
     // ---- experts: fc1 (gate and up in one pass, SwiGLU in the epilogue), fc2.  A shared expert as wide as the routed
-    // ones joins their launches as one more group: alone its 16 + 28 column blocks would occupy 22 % of the chip while
-    // a small batch streams its weights.  With stage times asked for it runs by itself, so that each of the reference's
+    // ones joins their launches as one more group: alone, its 16 and 28 column blocks (d 7168, f 2048) would occupy 22 and
+    // 38 % of the 74 CTA pairs while a small batch streams its weights.  With stage times asked for it runs by itself, so that each of the reference's
     // stages keeps a time of its own; the arithmetic is the same.
     const bool merged = fs == f && !metrics;
     const int* offsets = static_cast<const int*>(in->first_token_offset);

@@ -134,7 +134,10 @@ int rf_moe_ep_create(const RfMoeEpConfig* c, RfMoeEp** out) {
     ep->fs = c->d_expert * c->n_shared_experts;
     ep->push = c->push_results != 0 && c->world > 1;     // on one GPU nothing travels: plain fc2 + gathering combine
     // On 2 to 4 GPUs the dispatch runs by default as 32 copy-engine blocks beside the shared expert's GEMMs
-    // (measured: dispatch + shared expert 1.67 -> 1.25 ms on 4 GPUs, 2.90 -> 2.44 ms on 2).  On one GPU, where
+    // (measured: dispatch + shared expert 1.67 -> 1.25 ms on 4 GPUs, 2.90 -> 2.44 ms on 2; with the grouped GEMM on
+    // single CTAs.  On CTA pairs it has been timed beside the dispatch on one GPU only: of 8192 tokens, 32 dispatch
+    // blocks, the shared expert's two GEMMs end after 0.39 and 0.62 ms, the dispatch after 0.76, so no pair waits for
+    // an SM that the dispatch holds; blocks in clusters of two change those by 3, 2 and -1 %).  On one GPU, where
     // nothing crosses NVLink, it keeps every SM; on 8 it does too (measured: 3.75 against 3.73 ms per layer with the
     // partition; RF_MOE_EP_OPT_DISPATCH_BLOCKS selects it).
     ep->dispatch_blocks = (c->world > 1 && c->world <= 4) ? 32 : 0;

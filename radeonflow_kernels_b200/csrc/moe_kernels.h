@@ -17,8 +17,6 @@ cudaError_t moe_gather_rows_launch(const void* src, const int* row_map, int row_
                                    void* dst, int num_sms, cudaStream_t stream);
 cudaError_t moe_combine_launch(const void* y, const void* shared_out, const int* rev, const void* expanded_softmax,
                                int n_tokens, int top_k, int row_bytes, void* out, cudaStream_t stream);
-// dst[0] = a, dst[1] = b (a one-group offsets array written in stream order)
-cudaError_t moe_set_range_launch(int* dst, int a, int b, cudaStream_t stream);
 // Row ranges [offsets[g], offsets[g + 1]) -> list of row tiles for the grouped GEMM.  With alt_rows > 0 the list
 // starts with the tiles of one more group, number n_groups, of rows [0, alt_rows) of a matrix of its own (the
 // shared expert's).  At most alt_rows / kMoeTileRows + rows / kMoeTileRows + n_groups + 1 tiles.

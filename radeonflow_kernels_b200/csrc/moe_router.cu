@@ -5,10 +5,13 @@
 //   warp 1     MMA issuer: 4 x tcgen05.mma.kind::f16 (128 x N x 16) per stage, whole K accumulated in TMEM
 //   warps 4-11 epilogue of the previous tile while the next tile's MMAs run
 //
-// What bounds it: one tile's K loop, whose loads come from HBM, so the time is K steps x latency / stages in flight.  N is
-// the experts rounded up to 16, and the stages are as small as that allows and as many as fit: 32 experts take 9 stages of
-// 20 KB where boxes of 256 rows took 4 of 48.  128 tokens, K = 7168: 42.1 -> 32.0 us, 8192 tokens 49.0 -> 36.8.  (K is
-// not split over CTAs: sums in another order round single logits the other way, and a token then chooses another expert.)
+// What bounds it: one tile's K loop, at 0.25 to 0.33 us per 64-deep K step.  That depends little on what a step loads or
+// how many steps are in flight (K = 7168, 128 tokens; experts: KB per step, stages, us: 4: 17, 9, 28.6; 32: 20, 9, 31.7;
+// 128: 33, 6, 32.4; 256: 49, 4, 36.8), so it is neither one SM's load rate nor the loads' latency over the stages; which
+// hand-off of a step it is was not taken apart.  N is the experts rounded up to 16, and the stages are as small as that
+// allows and as many as fit: with boxes and MMAs of 256 rows for 32 experts 128 tokens took 42.1 us (now 32.0), 8192
+// tokens 49.0 (36.8).  (K is not split over CTAs: sums in another order round single logits the other way, and a token
+// then chooses another expert.)
 #include "ptx.cuh"
 #include "moe_kernels.h"
 
