@@ -258,7 +258,7 @@ struct WorkWalker<true> {
 // memory: each CTA leaves its fp32 tile in the stage ring, which its last K block has emptied, and sums its share of
 // the tile's rows over the cluster in ascending slice order (the order, and so the bits, of splitk_reduce_kernel).
 // That replaces the slices' round trip through memory and the second launch: 64 x 576 x 7168 in 8 slices takes 7.4 us
-// (8.6 before), 1024 x 512 x 7168 in 4 10.1 (11.5).  128-wide tiles only: 256-wide ones reach 22.2 us on 1024 x 1536 x
+// (8.6 before), 1024 x 512 x 7168 in 4 10.4 (11.5).  128-wide tiles only: 256-wide ones reach 22.2 us on 1024 x 1536 x
 // 7168 in 2 slices where 3 slices through memory take 18.3.
 template <class Cfg, bool STREAM_K = false, bool CLUSTER_K = false>
 __global__ void __launch_bounds__(Cfg::kThreads, 1)
