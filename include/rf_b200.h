@@ -79,9 +79,10 @@ void run(void *a, void *b, void *as, void *bs, void *c, int m, int n, int k, Per
 int rf_fp8_gemm(const void *a, const void *b, const float *as, const float *bs, void *c, int m, int n, int k,
                 int split_k, void *workspace, size_t workspace_bytes, rf_stream_t stream);
 
-/* Scratch bytes rf_fp8_gemm asks for at this shape and split (0 = library choice).  A plan with K slices asks for them
- * also where its slices meet in clusters and leave them unused (rf_fp8_gemm_kernel_launches): one answer with and without
- * a device, whatever clusters the device then holds.
+/* Scratch bytes that are enough for rf_fp8_gemm at this shape and split (0 = library choice), and for
+ * rf_fp8_gemm_colmajor[_fnuz], whose automatic plan may be another.  A plan with K slices asks for them also where its
+ * slices meet in clusters and leave them unused (rf_fp8_gemm_kernel_launches): one answer with and without a device,
+ * whatever clusters the device then holds.
  * Reference: init_workspace, src/gemm/gemm_launcher.cpp:30-36 (fixed 1.4 GB). */
 size_t rf_fp8_gemm_workspace_bytes(int m, int n, int k, int split_k);
 
@@ -108,7 +109,8 @@ int rf_fp8_gemm_work_pieces(int m, int n, int k, int block_n, int split_k, int n
  * The library starts with a built-in table for the benchmark shapes (RF_FP8_GEMM_NO_BUILTIN_PLANS=1 drops
  * it) and reads the file named by RF_FP8_GEMM_PLANS at first use.                                       */
 int rf_fp8_gemm_set_plan(int m, int n, int k, int block_n, int split_k);
-/* The plan the library would use (table entry or cost model; without a GPU that of a B200 with 148 SMs).  */
+/* The plan the library would use for row-major operands (table entry or cost model; without a GPU that of a
+ * B200 with 148 SMs).                                                                                     */
 int rf_fp8_gemm_get_plan(int m, int n, int k, int *block_n, int *split_k);
 /* Text file, one "m n k block_n split_k" per line, '#' comments (what `python -m
  * radeonflow_kernels_b200.tune` writes).  Returns the number of entries loaded, -1 if the file cannot be

@@ -69,36 +69,48 @@ int streamk_region(int m, int n, int k, int bn, int num_sms) {
     return sk;
 }
 
-// Whether the planner reckons with the K slices of `tiles` 128 x 128 tiles meeting in clusters: fewer clusters of 2 .. 8
-// CTAs than a B200 answers that it holds at once (with all 45 clusters of 3 in use 50 x 5696 x 2304 takes 9.5 us, one
+// Whether the planner reckons with the K slices of `tiles` 128 x 128 tiles meeting in clusters: the clusters of 2 .. 8
+// CTAs that a B200 answers that it holds at once, one of 3 less (with all 45 in use 50 x 5696 x 2304 takes 9.5 us, one
 // pass 7.7).  A table and not a question to the device, so that a plan is the same with and without one; whether a
 // launch runs in clusters is asked of its device (fp8_gemm_cluster_split).
 bool plan_in_clusters(int tiles, int splits) {
-    constexpr int kClusters[9] = {0, 0, 74, 45, 33, 26, 22, 15, 15};
-    return splits >= 2 && splits <= 8 && tiles < kClusters[splits];
+    constexpr int kClusters[9] = {0, 0, 74, 44, 33, 26, 22, 15, 15};
+    return splits >= 2 && splits <= 8 && tiles <= kClusters[splits];
 }
 
 // Cost model, in units of one 128-deep K block of a 128 x 128 tile (about 0.27 us where one round of tiles fits the
 // chip: 64 x 576 x 7168 takes 17.7, 12.8, 8.9, 7.4 us with 56, 28, 14, 7 K blocks per CTA): rounds of tiles over the
-// SMs x (K blocks per slice + fixed per-tile cost), plus, for split-K, either the cluster's exchange (3.0 us) or the fp32
-// slices and the second launch (3.2 us; with less than one 32-row box of rows 5.7; behind the longer epilogue of a
-// 256-wide tile 4.9).  The constants are those that lose least over 2009 shapes of up to 300 tiles, each timed under every
-// plan in a CUDA graph: 1.2 % on the geometric mean against the fastest plan.  (With 2.5 us for every second launch it was
-// 3.3 %: 4 x 6080 x 2176 was split in 3 slices, 9.7 us where a plain pass takes 7.6, and 50 x 4480 x 4864 in 8 wide
-// ones, 11.7 us where 4 of 128 take 9.4.)
-GemmPlan plan_for(int m, int n, int k, int num_sms, int bn, int forced_split) {
+// SMs x (K blocks per slice + fixed per-tile cost), plus, for split-K, either the cluster's exchange or the fp32 slices
+// (those of one round stay in L2) and the second launch.
+struct PlanCosts {
+    double wide_block;        // one K block of a 128 x 256 tile with at most one tile per SM, where latency decides
+    double exchange;          // of slices that meet in a cluster
+    double second_launch;     // 128-wide tiles ...
+    double few_rows;          // ... of fewer rows than one 32-row store box
+    double wide_launch;       // behind the longer epilogue of a 256-wide tile
+    double slice_rate;        // bytes / s
+    int short_blocks;         // one tile per SM with at most so many K blocks is not split through memory
+};
+// Row-major operands: the constants that lose least over 2009 shapes of up to 300 tiles, each timed under every plan in a
+// CUDA graph, 1.2 % on the geometric mean against the fastest plan.  (With the row below it was 3.3 %: 4 x 6080 x 2176 was
+// split in 3 slices, 9.7 us where one pass takes 7.6, and 50 x 4480 x 4864 in 8 wide ones, 11.7 us where 4 of 128 take
+// 9.4.)  A call of two launches keeps the host busy for about 9.4 us, hence short_blocks: called in a loop, one pass
+// against 3 slices through memory, 50 x 5888 x 2560 8.4 / 9.5 us, 64 x 5888 x 3072 9.3 / 9.4, 64 x 5888 x 3712 10.6 / 9.4.
+constexpr PlanCosts kRowMajorCosts = {1.4, 11.0, 12.0, 21.0, 18.0, 16.0e12, 24};
+// The reference's layout: kernels of its own, behind a conversion pass that keeps the GPU busy while the host launches.
+// 929 shapes, 1.7 % with these, 1.9 % with the row above (2000 x 704 x 5504 in 3 wide slices 24.3 us, in one
+// pass 30.6).
+constexpr PlanCosts kRefLayoutCosts = {1.5, 10.0, 9.3, 9.3, 9.3, 12.0e12, 0};
+
+GemmPlan plan_for(int m, int n, int k, int num_sms, int bn, int forced_split, const PlanCosts& c) {
     const int tr = rf::gemm_tile_rows(bn), tc = rf::gemm_tile_cols(bn);
     const int tiles = ((m + tr - 1) / tr) * ((n + tc - 1) / tc);
     const int kb = k / kBlockK;
     if (rf::gemm_is_pair(bn)) num_sms /= 2;     // work items go to CTA pairs
     // relative time of one K block of one work item, from in-kernel cycle counts
-    // (128 x 128: ~620 cycles, 128 x 256: ~790, CTA pair 256 x 256: ~925); with at most one item per SM, where latency
-    // and not the shared pipes decide, a 128 x 256 tile takes 0.38 us a K block
+    // (128 x 128: ~620 cycles, 128 x 256: ~790, CTA pair 256 x 256: ~925)
     const double wide = bn == 512 ? 1.5 : (bn == 256 ? 1.25 : (bn == 384 ? 0.8 : 1.0));
-    // One 128 x 128 tile per SM, its K loop no longer than the host takes for two launches (about 9.4 us).  Called in a
-    // loop, one pass against 3 slices through memory: 50 x 5888 x 2560 8.4 / 9.5 us, 64 x 5888 x 3072 9.3 / 9.4, 64 x
-    // 5888 x 3712 10.6 / 9.4.
-    const bool short_pass = kb + 4 <= 28 && ((m + 127) / 128) * ((n + 127) / 128) <= num_sms;
+    const bool short_pass = kb <= c.short_blocks && ((m + 127) / 128) * ((n + 127) / 128) <= num_sms;
     GemmPlan best{bn, 1, 1e30};
     for (int s = 1; s <= 8; ++s) {
         if (forced_split > 0 && s != forced_split) continue;
@@ -106,14 +118,14 @@ GemmPlan plan_for(int m, int n, int k, int num_sms, int bn, int forced_split) {
         if (s > kb) break;
         const int rounds = (tiles * s + num_sms - 1) / num_sms;
         const int kb_per = (kb + s - 1) / s;
-        const double tile_w = bn == 256 && rounds == 1 ? 1.4 : wide;
+        const double tile_w = bn == 256 && rounds == 1 ? c.wide_block : wide;
         double cost = (double)rounds * (kb_per * tile_w + 4.0);
         if (s > 1 && bn == 128 && plan_in_clusters(tiles, s)) {
-            cost += 11.0;
+            cost += c.exchange;
         } else if (s > 1) {
             if (short_pass && forced_split <= 0) continue;
-            const double bytes = 8.0 * s * (double)m * n + 2.0 * (double)m * n;      // (slices of one round stay in L2)
-            cost += bytes / 16.0e12 / 0.27e-6 + (bn == 128 ? (m < 32 ? 21.0 : 12.0) : 18.0);
+            const double bytes = 8.0 * s * (double)m * n + 2.0 * (double)m * n;
+            cost += bytes / c.slice_rate / 0.27e-6 + (bn != 128 ? c.wide_launch : m < 32 ? c.few_rows : c.second_launch);
         }
         if (cost < best.cost) best = GemmPlan{bn, s, cost};
     }
@@ -121,19 +133,19 @@ GemmPlan plan_for(int m, int n, int k, int num_sms, int bn, int forced_split) {
     return best;
 }
 
-GemmPlan choose_plan_inner(int m, int n, int k, int num_sms, int forced_split) {
+GemmPlan choose_plan_inner(int m, int n, int k, int num_sms, int forced_split, const PlanCosts& c) {
     const int fb = forced_block_n();
-    if (fb) return plan_for(m, n, k, num_sms, fb, forced_split);
+    if (fb) return plan_for(m, n, k, num_sms, fb, forced_split, c);
     // a measured entry for this exact shape beats the model (the caller's explicit split still wins)
     int tbn = 0, tsplits = 0;
     if (forced_split <= 0 && rf::tuned_plan_lookup(m, n, k, &tbn, &tsplits)) return GemmPlan{tbn, tsplits, 0.0};
-    GemmPlan p128 = plan_for(m, n, k, num_sms, 128, forced_split);
-    GemmPlan p256 = plan_for(m, n, k, num_sms, 256, forced_split);
+    GemmPlan p128 = plan_for(m, n, k, num_sms, 128, forced_split, c);
+    GemmPlan p256 = plan_for(m, n, k, num_sms, 256, forced_split, c);
     // Wide tiles halve the A traffic and the MMA instruction count per FLOP; prefer them unless
     // they cost noticeably more rounds (ragged N such as 576, or too few tiles).
     GemmPlan best = p256.cost <= p128.cost * 1.02 ? p256 : p128;
     if (pair_config_enabled()) {
-        GemmPlan pp = plan_for(m, n, k, num_sms, 512, forced_split);
+        GemmPlan pp = plan_for(m, n, k, num_sms, 512, forced_split, c);
         if (pp.cost < best.cost) best = pp;
     }
     // Stream-K instead of a plain single pass, in K blocks of the chosen tile: a plain pass takes
@@ -157,8 +169,9 @@ GemmPlan choose_plan_inner(int m, int n, int k, int num_sms, int forced_split) {
 }
 
 // forced_split: > 0 = that many K slices, kStreamK = stream-K, 0 = the library's choice.
-GemmPlan choose_plan(int m, int n, int k, int num_sms, int forced_split) {
-    GemmPlan plan = choose_plan_inner(m, n, k, num_sms, forced_split == kStreamK ? 1 : forced_split);
+GemmPlan choose_plan(int m, int n, int k, int num_sms, int forced_split, bool mn_major = false) {
+    const PlanCosts& costs = mn_major ? kRefLayoutCosts : kRowMajorCosts;
+    GemmPlan plan = choose_plan_inner(m, n, k, num_sms, forced_split == kStreamK ? 1 : forced_split, costs);
     if (forced_split == kStreamK) plan.splits = kStreamK;
     if (forced_split == 0) {
         const int ov = streamk_override();
@@ -199,8 +212,9 @@ int gemm_impl(const void* a, const void* b, const float* as, const float* bs, vo
     if (split_k > kb) split_k = kb;
     if (split_k > kMaxSplits) split_k = kMaxSplits;
     if (split_k < kStreamK) return RF_ERR_BAD_SHAPE;
-    GemmPlan plan = choose_plan(m, n, k, st->num_sms, split_k);
-    if (mn_major && rf::gemm_is_pair(plan.block_n)) plan = plan_for(m, n, k, st->num_sms, 256, split_k > 0 ? split_k : 0);
+    GemmPlan plan = choose_plan(m, n, k, st->num_sms, split_k, mn_major);
+    if (mn_major && rf::gemm_is_pair(plan.block_n))
+        plan = plan_for(m, n, k, st->num_sms, 256, split_k > 0 ? split_k : 0, kRefLayoutCosts);
     // stream-K serves the row-major single-destination GEMM; elsewhere such a plan runs as a plain pass
     if (plan.splits == kStreamK && (mn_major || n_dest > 1 || rf::gemm_is_pair(plan.block_n))) plan.splits = 1;
     const int bn = plan.block_n;
@@ -407,9 +421,15 @@ size_t rf_fp8_gemm_workspace_bytes(int m, int n, int k, int split_k) {
     const int kb = k / kBlockK;
     if (split_k > kb) split_k = kb;
     if (split_k > kMaxSplits) split_k = kMaxSplits;
-    const GemmPlan plan = choose_plan(m, n, k, num_sms, split_k);
-    if (plan.splits == kStreamK) return rf::gemm_streamk_bytes(plan.block_n, num_sms);
-    return plan.splits > 1 ? (size_t)plan.splits * m * n * sizeof(float) : 0;
+    // (the reference's layout may have another plan, and runs a stream-K one as a plain pass)
+    size_t bytes = 0;
+    for (bool mn_major : {false, true}) {
+        const GemmPlan plan = choose_plan(m, n, k, num_sms, split_k, mn_major);
+        size_t need = plan.splits > 1 ? (size_t)plan.splits * m * n * sizeof(float) : 0;
+        if (plan.splits == kStreamK && !mn_major) need = rf::gemm_streamk_bytes(plan.block_n, num_sms);
+        if (need > bytes) bytes = need;
+    }
+    return bytes;
 }
 
 int rf_fp8_gemm(const void* a, const void* b, const float* as, const float* bs, void* c, int m, int n, int k,

@@ -175,3 +175,29 @@ def test_short_k_two_slab_configuration_with_ragged_tiles(rf_lib, m, n, k):
         assert ok, (n_bad, max_err)
     finally:
         rf_lib.rf_fp8_gemm_set_plan(m, n, k, 0, 0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,n,k", [(2000, 704, 5504), (304, 576, 1024), (48, 4864, 2176)])
+def test_workspace_bytes_serve_the_reference_layout_too(rf_lib, m, n, k):
+    """The reference-layout entry may split where the row-major one does not; a caller's workspace of the size that
+    rf_fp8_gemm_workspace_bytes names is enough for either."""
+    import torch
+    from oracle import fp8_gemm as o
+    from radeonflow_kernels_b200 import gemm as G
+    from tests.helpers import canary_intact, canary_output, gemm_device_inputs
+    a, b, a_s, b_s = o.generate_input(m, n, k, 4)
+    size = rf_lib.rf_fp8_gemm_workspace_bytes(m, n, k, 0)
+    ref = o.fp8_gemm(a, b, a_s, b_s)
+    for entry, ops in ((rf_lib.rf_fp8_gemm_colmajor, [np.ascontiguousarray(t.T) for t in (a, b, a_s, b_s)]),
+                       (rf_lib.rf_fp8_gemm, [a, b, a_s, b_s])):
+        dev = gemm_device_inputs(*ops)
+        ws = torch.full((size + 64,), 0x5A, dtype=torch.uint8, device="cuda:0")
+        full, c = canary_output(m, n)
+        split = (0,) if entry is rf_lib.rf_fp8_gemm else ()
+        assert entry(*[t.data_ptr() for t in dev], c.data_ptr(), m, n, k, *split, ws.data_ptr(), size, None) == 0
+        torch.cuda.synchronize()
+        assert G.device_status() == 0 and canary_intact(full, m, n)
+        assert bool((ws[size:] == 0x5A).all())
+        ok, n_bad, max_err = o.check(c.view(torch.uint16).cpu().numpy(), ref)
+        assert ok, (n_bad, max_err)
