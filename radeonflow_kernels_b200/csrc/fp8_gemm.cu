@@ -8,10 +8,9 @@
 // One persistent CTA per SM, warp-specialised:
 //   warp 0      TMA producer: A [128 x 128 B] and B [BN x 128 B] tiles, 128-byte
 //               swizzle, into a STAGES-deep shared-memory ring (mbarrier tx counts)
-//   warps 1, 2  MMA issuers, alternating K blocks: per 128-deep K block, 4 x
-//               tcgen05.mma.kind::f8f6f4 (K = 32 each) into one of 512/BN TMEM
-//               accumulator buffers, then ONE tcgen05.commit that publishes the
-//               buffer (the epilogue, which observes it, frees the smem stage)
+//   warp 1      MMA issuer: per 128-deep K block, 4 x tcgen05.mma.kind::f8f6f4
+//               (K = 32 each) into one of 512/BN TMEM accumulator buffers, then a
+//               tcgen05.commit that publishes the buffer
 //   warps 4..   epilogue: tcgen05.ld the K block's fp32 partial sums, scale by
 //               the exact fp32 product a_s*b_s and add into a register
 //               accumulator (packed fma.rn.f32x2) while the next K blocks' MMAs run
@@ -24,6 +23,7 @@
 // (src/gemm/gemm_kernel.cpp:173-207).
 #include "ptx.cuh"
 #include "fp8_gemm.h"
+#include "fp8_tiles.cuh"
 
 #include <atomic>
 #include <cstdio>
@@ -58,37 +58,30 @@ constexpr int UMMA_K = 32;       // K per tcgen05.mma for 8-bit operands
 constexpr int NUM_NON_EPI_WARPS = 4;
 constexpr int kMaxClusterSlices = 8;     // the portable cluster size
 
-// TWO_CTA: the tile is 256 x BN per CTA PAIR (2-CTA cluster): each CTA loads its own 128 rows of A and
-// half of the B rows, the leader CTA issues cta_group::2 MMAs (M = 256) whose accumulator rows
-// 0-127 / 128-255 land in the two CTAs' TMEM.  Per SM and K block this moves 32 KB through shared
-// memory each way instead of 48 KB; measured, it is still slower than the 1-CTA 128 x 256 tile (the
-// epilogue's promotion work, not shared memory, bounds both), so it is selectable but not the default.
 // MN_MAJOR: operands stored [k][m] and [k][n] (M / N contiguous), the reference's physical layout
 // (src/gemm/gemm_kernel_legacy.cpp:264-268); consumed directly as MN-major UMMA operands, so the
 // reference's transpose pass (src/gemm/gemm_launcher.cpp:55-56) has no counterpart here.
 // SLABS: store slabs per epilogue warp.  With two, the second 64-column chunk of a tile is staged while the
 // TMA is still reading the first; worth its 32 KB of shared memory (one pipeline stage fewer) only when K is
 // short and the per-tile store is a large share of the tile's time.
-template <int BN, int STAGES, bool TWO_CTA = false, bool MN_MAJOR = false, int SLABS = 1>
+template <int BN, int STAGES, bool MN_MAJOR = false, int SLABS = 1>
 struct GemmCfg {
     static constexpr int kBN = BN;
     static constexpr int kStages = STAGES;
-    static constexpr bool kTwoCta = TWO_CTA;
     static constexpr bool kMnMajor = MN_MAJOR;
-    static_assert(!(TWO_CTA && MN_MAJOR), "the CTA-pair configuration is K-major only");
-    static constexpr int kBRows = TWO_CTA ? BN / 2 : BN;       // rows of B this CTA loads per K block
     static constexpr int kEpiGroups = 2;                       // column groups, 4 warps each
     static constexpr int kColsPerThread = BN / kEpiGroups;     // 64 or 128: one scale block at most
     static constexpr int kEpiWarps = 4 * kEpiGroups;
     static constexpr int kThreads = 32 * (NUM_NON_EPI_WARPS + kEpiWarps);   // 384
     static constexpr int kABytes = BM * BK;
-    static constexpr int kBBytes = kBRows * BK;
+    static constexpr int kBBytes = BN * BK;
     static constexpr int kStageBytes = kABytes + kBBytes;
+    static constexpr bool kCommitFreesStage = BN == 128;      // who gives a stage back: the MMAs' commit, or the epilogue
     static constexpr int kTmemBufs = 512 / BN;                // accumulator buffers in flight
     static constexpr int kTmemCols = kTmemBufs * BN;          // all 512 TMEM columns
-    // full / empty / peer-full per stage, full / empty per accumulator buffer, the two stream-K barriers, the
-    // TMEM address slot (16 bytes)
-    static constexpr int kBarBytes = (3 * STAGES + 2 * kTmemBufs + 2) * 8 + 16;
+    // full / empty per stage, full / empty per accumulator buffer, the two stream-K barriers, the TMEM address slot
+    // (16 bytes)
+    static constexpr int kBarBytes = (2 * STAGES + 2 * kTmemBufs + 2) * 8 + 16;
     static constexpr int kSlabBytes = 32 * 128;               // one slab: 32 rows x 128 B, swizzled
     static constexpr int kSlabs = SLABS;                      // slabs per epilogue warp
     static_assert(SLABS == 1 || SLABS == 2, "one or two store slabs per warp");
@@ -96,8 +89,11 @@ struct GemmCfg {
         STAGES * kStageBytes + kEpiWarps * kSlabs * kSlabBytes + kBarBytes + 1024;       // + alignment slack
     // The epilogue (64 or 128 accumulators per thread plus staging) wants more than the 168 registers a
     // 384-thread CTA starts with, the producer warpgroup far fewer: registers are rebalanced after set-up
-    // (128 * kRegsLo + 256 * kRegsHi <= 64512, the CTA's allocation at 168 per thread).  The split is chosen by
-    // measurement on the 18-shape sweep.
+    // (128 * kRegsLo + 256 * kRegsHi <= 64512, the CTA's allocation at 168 per thread).  The splits are measured ones: at
+    // most others ptxas copies accumulators inside the K loop, without a spill to show for it.  256 wide, 6144 x 4608 x
+    // 7168: 64 / 216 242 us, 72 / 216 247, 88 / 208 224; 56 / 224, 104 / 200 and 120 / 192 176, of which the last is the
+    // fastest of the three on short calls.  128 wide, 68 x 6464 x 3456 in 2 slices: 120 / 192 9.8, no rebalancing 10.1,
+    // 56 / 224 9.5.
     static constexpr bool kRebalanceRegs = true;
 #if defined(RF_REGS_LO) && defined(RF_REGS_HI)
     static constexpr int kRegsLo = RF_REGS_LO, kRegsHi = RF_REGS_HI;
@@ -105,19 +101,12 @@ struct GemmCfg {
     static constexpr int kRegsLo = kColsPerThread > 64 ? 40 : 104;
     static constexpr int kRegsHi = kColsPerThread > 64 ? 232 : 200;
 #else
-    // (56 / 224 for the row-major one-slab configurations, 120 / 192 for the others; 88 / 208 and 72 / 216 run the
-    // sweep 17 % and 27 % slower: ptxas allocates the K loop differently at every split)
-    static constexpr bool kWideSplit = !TWO_CTA && !MN_MAJOR && SLABS == 1;
-    static constexpr int kRegsLo = kWideSplit ? 56 : 120, kRegsHi = kWideSplit ? 224 : 192;
+    static constexpr int kRegsLo = BN == 128 ? 56 : 120, kRegsHi = BN == 128 ? 224 : 192;
 #endif
     static_assert(128 * kRegsLo + 256 * kRegsHi <= 64512 && kRegsLo % 8 == 0 && kRegsHi % 8 == 0, "register split");
     static_assert(kColsPerThread == 64 || kColsPerThread == 128, "epilogue handles 64 or 128 columns per thread");
     static_assert(kTmemCols == 512, "TMEM columns: power of two, at most 512");
     static_assert(kSmemBytes <= 227 * 1024, "shared memory budget");
-};
-
-struct TileCoord {
-    int m_blk, n_blk;
 };
 
 // OR of the words the e4m3fnuz conversion pass left: 1 = A, 2 = B holds a byte that reads differently as e4m3fn.
@@ -132,34 +121,6 @@ __device__ __forceinline__ uint32_t fnuz_special(const uint32_t* words) {
     }
     return __reduce_or_sync(0xffffffffu, v);
 }
-
-// Tile number -> tile.  Consecutive tiles walk down M inside a band of GROUP_M row blocks before moving to
-// the next column block, so the CTAs that run concurrently share B tiles (and A bands) in L2.
-__device__ __forceinline__ TileCoord decode_tile(int tile, int tiles_m, int tiles_n) {
-    // (This runs once per tile in every role, on the epilogue's critical path between two tiles: one integer
-    // division, and shifts for the full bands.  Measured: the earlier form with five divisions, together with two
-    // 64-bit divisions for the K range, cost the epilogue about 1400 cycles per tile, the present one 600.)
-    constexpr int GROUP_M = 8;
-    TileCoord t;
-    const int group = GROUP_M * tiles_n;
-    const int band = tile / group;
-    const int first_m = band * GROUP_M;
-    const int band_rows = min(GROUP_M, tiles_m - first_m);
-    const int in_band = tile - band * group;
-    if (band_rows == GROUP_M) {
-        t.m_blk = first_m + (in_band & (GROUP_M - 1));
-        t.n_blk = in_band >> 3;
-    } else {
-        t.n_blk = in_band / band_rows;
-        t.m_blk = first_m + in_band - t.n_blk * band_rows;
-    }
-    return t;
-}
-
-// One stretch of work of a CTA: K blocks [kb0, kb1) of work item `item` = tile * splits + K-slice number.
-struct Piece {
-    int item, kb0, kb1;
-};
 
 // First K-block unit of CTA j's share of the stream-K region (`total` units over `n_units` CTAs).
 __host__ __device__ __forceinline__ int sk_share_begin(long long total, int j, int n_units) {
@@ -182,10 +143,8 @@ __host__ __device__ __forceinline__ bool sk_contributes(long long total, int j, 
 // First tile of the stream-K region.
 __host__ __device__ __forceinline__ int sk_tile0(const GemmParams& p) { return p.tiles_m * p.tiles_n - p.sk_tiles; }
 
-// The sequence of pieces a CTA works through; producer, MMA issuers and epilogue each walk their own copy.
+// The walker of plain launches (PlainWalker) and of stream-K launches.
 //
-// Plain launches: work items unit, unit + n_units, ... (a work item is a tile, or one K slice of a tile; the K
-// slices of one tile are adjacent).
 // Stream-K launches (p.sk_tiles > 0): the LAST p.sk_tiles tiles form a region whose K blocks, numbered
 // tile-major, are cut into n_units equal contiguous shares, so that no SM idles in a ragged last wave.  A CTA
 // takes its share from the TOP down (so a tile that continues in the next CTA's share is started first and
@@ -194,32 +153,11 @@ __host__ __device__ __forceinline__ int sk_tile0(const GemmParams& p) { return p
 // flag at the very beginning of its run) and the upper CTA, which holds the tile's last K block, the owner
 // (it adds the slots of the contributors, all of LOWER block index and long finished with them, and stores
 // the tile).  Waiting only ever goes to lower block indices, which are scheduled no later than the waiter.
+// (p.splits == 1, so a work item is a tile.)
 template <bool STREAM_K>
-struct WorkWalker;
-
-// Plain launches.  (One register of state: the epilogue's register budget is tight and its allocation fragile.)
-template <>
-struct WorkWalker<false> {
-    int w;                     // the work item drawn last
-    __host__ __device__ __forceinline__ WorkWalker(const GemmParams&, int unit, int n_units, int) { w = unit - n_units; }
-    __host__ __device__ __forceinline__ bool next(Piece& pc, const GemmParams& p, int n_units, int kb_total) {
-        w += n_units;
-        if (w >= p.tiles_m * p.tiles_n * p.splits) return false;
-        pc.item = w;
-        if (p.splits == 1) {
-            pc.kb0 = 0;
-            pc.kb1 = kb_total;
-        } else {
-            // (k / 128 < 2^24 and splits <= 64: the products fit 32 bits)
-            const int split = w % p.splits;
-            pc.kb0 = kb_total * split / p.splits;
-            pc.kb1 = kb_total * (split + 1) / p.splits;
-        }
-        return true;
-    }
+struct WorkWalker : PlainWalker {
+    using PlainWalker::PlainWalker;
 };
-
-// Stream-K launches (p.splits == 1, so a work item is a tile).
 template <>
 struct WorkWalker<true> {
     int u_lo, u_hi;            // stream-K units of this CTA not yet done: [u_lo, u_hi), taken from the top
@@ -269,7 +207,7 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
     constexpr int STAGES = Cfg::kStages;
     constexpr int CPT = Cfg::kColsPerThread;
     constexpr int NBUF = Cfg::kTmemBufs;
-    static_assert(!CLUSTER_K || (BN == 128 && !Cfg::kTwoCta && !STREAM_K), "cluster split-K: 128 x 128 tiles");
+    static_assert(!CLUSTER_K || (BN == 128 && !STREAM_K), "cluster split-K: 128 x 128 tiles");
 
     extern __shared__ uint8_t smem_raw[];
     // 128-byte-swizzled tiles need 1024-byte alignment.
@@ -280,29 +218,21 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
     auto empty_bar = [&](int s) { return bar_base + 8u * (STAGES + s); };
     auto tmem_full_bar = [&](int b) { return bar_base + 8u * (2 * STAGES + b); };
     auto tmem_empty_bar = [&](int b) { return bar_base + 8u * (2 * STAGES + NBUF + b); };
-    auto peer_full_bar = [&](int s) { return bar_base + 8u * (2 * STAGES + 2 * NBUF + s); };   // leader only
     // stream-K: "this CTA's partial sums are stored" (8 epilogue warps -> warp 3) and "the partial sums this CTA's
     // owner piece needs have arrived" (warp 3 -> epilogue warps); each is used at most once per launch
-    const uint32_t sk_stored_bar = bar_base + 8u * (3 * STAGES + 2 * NBUF);
+    const uint32_t sk_stored_bar = bar_base + 8u * (2 * STAGES + 2 * NBUF);
     const uint32_t sk_ready_bar = sk_stored_bar + 8u;
-    const uint32_t tmem_slot = bar_base + 8u * (3 * STAGES + 2 * NBUF + 2);
+    const uint32_t tmem_slot = bar_base + 8u * (2 * STAGES + 2 * NBUF + 2);
     uint32_t* tmem_slot_ptr =
         reinterpret_cast<uint32_t*>(smem_raw + (tmem_slot - smem_u32(smem_raw)));
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
-    constexpr bool TWO = Cfg::kTwoCta;
     // The next kernel in the stream may be scheduled onto SMs as this grid's CTAs leave them; it blocks in
     // its own griddep_wait() until this grid has completed.
     griddep_launch_dependents();
-#ifdef RF_SINGLE_ISSUE
-    constexpr bool kDualIssue = false;
-#else
-    constexpr bool kDualIssue = NBUF % 2 == 0;
-#endif
-    const uint32_t cta_rank = TWO ? cluster_ctarank() : 0u;      // 0 = leader of the pair
-    const int unit = TWO ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;          // work-loop index
-    const int unit_stride = TWO ? (int)(gridDim.x >> 1) : (int)gridDim.x;
+    const int unit = (int)blockIdx.x;          // work-loop index
+    const int unit_stride = (int)gridDim.x;
 
     if (threadIdx.x == 0) {
         tma_prefetch_desc(&tma_a);
@@ -312,30 +242,22 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
             mbar_init(full_bar(s), 1);
             mbar_init(empty_bar(s), 1);
         }
-        for (int s = 0; s < STAGES; ++s) mbar_init(peer_full_bar(s), 1);
         if (STREAM_K) {
             mbar_init(sk_stored_bar, Cfg::kEpiWarps);
             mbar_init(sk_ready_bar, 1);
         }
         for (int b = 0; b < NBUF; ++b) {
             mbar_init(tmem_full_bar(b), 1);
-            // in a CTA pair the leader's barrier collects the epilogue warps of both CTAs
-            mbar_init(tmem_empty_bar(b), TWO ? 2 * Cfg::kEpiWarps : Cfg::kEpiWarps);
+            mbar_init(tmem_empty_bar(b), Cfg::kEpiWarps);
         }
         mbar_fence_init();
     }
     if (warp == 1) {
-        if (TWO) {
-            tmem_alloc_2cta(tmem_slot, Cfg::kTmemCols);
-            tmem_relinquish_2cta();
-        } else {
-            tmem_alloc(tmem_slot, Cfg::kTmemCols);
-            tmem_relinquish();
-        }
+        tmem_alloc(tmem_slot, Cfg::kTmemCols);
+        tmem_relinquish();
     }
     tc_fence_before();
     __syncthreads();
-    if (TWO) cluster_sync_all();     // both CTAs' barriers exist before any remote arrive or multicast commit
     tc_fence_after();
     const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(tmem_slot_ptr);
     // Barriers, TMEM and descriptors are set up; everything below reads or writes global memory that the
@@ -348,9 +270,10 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
     // Register split after set-up: the 4 producer / MMA warps shrink to kRegsLo, the 8 epilogue warps grow
     // to kRegsHi.
     if (Cfg::kRebalanceRegs) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(Cfg::kRegsLo));
-    // Producer and MMA warps keep all 32 lanes in the loops (warp-uniform control
-    // flow, so descriptors and addresses live in uniform registers) and elect one
-    // lane only for the instructions that must be issued once.
+    // Producer and MMA issuer each run on one lane: a step of theirs is a serial chain, and every instruction of it
+    // queues behind those of the epilogue warps on the same scheduler.  (1024 x 1536 x 7168 in one pass of 128-wide tiles
+    // 18.3 us as whole warps that vote and elect at every step, two of them issuing MMAs in turn; now 17.8.  1024 x 4096 x
+    // 512: 6.36, now 6.09.)
     if (warp == 0) {
         // ------------------------------------------------------ TMA producer
         uint32_t it = 0;  // running K-block counter across work items
@@ -365,21 +288,20 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
             if (special & 1u) map_a = &dests.m[0];
             if (special & 2u) map_b = &dests.m[1];
         }
-        WorkWalker<STREAM_K> walk(p, unit, unit_stride, kb_total);
-        Piece pc;
-        while (ok && walk.next(pc, p, unit_stride, kb_total)) {
-            const TileCoord t = decode_tile(p.splits == 1 ? pc.item : pc.item / p.splits, p.tiles_m, p.tiles_n);
-            // rows of A and of B this CTA fetches (a CTA pair splits both between its two CTAs)
-            const int a_row0 = TWO ? (t.m_blk * 2 + (int)cta_rank) * BM : t.m_blk * BM;
-            const int b_row0 = t.n_blk * BN + (TWO ? (int)cta_rank * Cfg::kBRows : 0);
-            for (int kb = pc.kb0; kb < pc.kb1; ++kb, ++it) {
-                const int s = it % STAGES;
-                const uint32_t ph = (it / STAGES) & 1;
-                { RF_STAT_BEGIN();
-                ok = __all_sync(0xffffffffu, mbar_wait(empty_bar(s), ph ^ 1, p.status, kErrProducerWait, p.launch_tag));
-                RF_STAT_END(w_empty); }
-                if (!ok) break;
-                if (elect_one()) {
+        if (elect_one()) {
+            WorkWalker<STREAM_K> walk(p, unit, unit_stride, kb_total);
+            Piece pc;
+            while (ok && walk.next(pc, p, unit_stride, kb_total)) {
+                const TileCoord t = decode_tile(p.splits == 1 ? pc.item : pc.item / p.splits, p.tiles_m, p.tiles_n);
+                const int a_row0 = t.m_blk * BM;
+                const int b_row0 = t.n_blk * BN;
+                for (int kb = pc.kb0; kb < pc.kb1; ++kb, ++it) {
+                    const int s = it % STAGES;
+                    const uint32_t ph = (it / STAGES) & 1;
+                    { RF_STAT_BEGIN();
+                    ok = mbar_wait(empty_bar(s), ph ^ 1, p.status, kErrProducerWait, p.launch_tag);
+                    RF_STAT_END(w_empty); }
+                    if (!ok) break;
                     mbar_expect_tx(full_bar(s), Cfg::kStageBytes);
                     const uint32_t sa = smem_base + s * Cfg::kStageBytes;
                     if (Cfg::kMnMajor) {
@@ -394,19 +316,13 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
                         tma_load_2d(sa + Cfg::kABytes, &tma_b, full_bar(s), kb * BK, b_row0);
                     }
                 }
-                __syncwarp();
             }
+            RF_STAT_FLUSH(0, w_empty);
         }
-        if (lane == 0) { RF_STAT_FLUSH(0, w_empty); }
-    } else if (warp == 1 || (kDualIssue && warp == 2)) {
-        // ------------------------------------------------------- MMA issuers
-        // Issuing one K block (two barrier waits, four MMAs, one commit) is a serial chain of a few
-        // hundred cycles in a single thread, about as long as the MMAs take to execute.  Two warps on
-        // different schedulers therefore alternate K blocks: even blocks (and the even TMEM buffers)
-        // belong to warp 1, odd ones to warp 2.  Blocks are independent (separate accumulator buffers
-        // and smem stages), so no ordering between the two issuers is needed.
-        const uint32_t my_parity = (uint32_t)(warp - 1);
-        constexpr uint32_t idesc = make_idesc(TWO ? 2 * BM : BM, BN, /*e4m3*/ 0, /*e4m3*/ 0,
+        __syncwarp();
+    } else if (warp == 1) {
+        // -------------------------------------------------------- MMA issuer
+        constexpr uint32_t idesc = make_idesc(BM, BN, /*e4m3*/ 0, /*e4m3*/ 0,
                                               Cfg::kMnMajor ? 1 : 0, Cfg::kMnMajor ? 1 : 0);
         // descriptor advance per MMA (K = 32): 32 bytes inside the swizzled row for K-major operands,
         // 32 K-rows of 128 bytes for MN-major ones (address field is in 16-byte units)
@@ -414,65 +330,46 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
         uint32_t it = 0;
         bool ok = true;
         long long w_tmem = 0, w_full = 0, w_issue = 0; (void)w_tmem; (void)w_full; (void)w_issue;
-        WorkWalker<STREAM_K> walk(p, unit, unit_stride, kb_total);
-        Piece pc;
-        while (ok && walk.next(pc, p, unit_stride, kb_total)) {
-            for (int kb = pc.kb0; kb < pc.kb1; ++kb, ++it) {
-                const int s = it % STAGES;
-                const uint32_t ph = (it / STAGES) & 1;
-                const int buf = it % NBUF;
-                const uint32_t bph = (it / NBUF) & 1;
-                if (kDualIssue && (it & 1u) != my_parity) continue;
-                if (TWO && cta_rank != 0) {
-                    // Second CTA of the pair: it issues no MMA.  This warp relays "my stage has landed"
-                    // to the leader (a TMA load can only signal a barrier of the CTA it writes to).
-                    ok = __all_sync(0xffffffffu, mbar_wait(full_bar(s), ph, p.status, kErrMmaWaitFull, p.launch_tag));
+        if (elect_one()) {
+            WorkWalker<STREAM_K> walk(p, unit, unit_stride, kb_total);
+            Piece pc;
+            while (ok && walk.next(pc, p, unit_stride, kb_total)) {
+                for (int kb = pc.kb0; kb < pc.kb1; ++kb, ++it) {
+                    const int s = it % STAGES;
+                    const uint32_t ph = (it / STAGES) & 1;
+                    const int buf = it % NBUF;
+                    const uint32_t bph = (it / NBUF) & 1;
+                    { RF_STAT_BEGIN();
+                    ok = mbar_wait(tmem_empty_bar(buf), bph ^ 1, p.status, kErrMmaWaitTmem, p.launch_tag);
+                    RF_STAT_END(w_tmem); }
                     if (!ok) break;
-                    // (no memory ordering needed: the stage was written by the TMA and is read by the
-                    // tensor core, both through the async proxy; the barrier flip means the bytes landed)
-                    if (elect_one()) mbar_arrive_cluster_relaxed(mapa_cluster(peer_full_bar(s), 0));
-                    __syncwarp();
-                    continue;
-                }
-                { RF_STAT_BEGIN();
-                ok = __all_sync(0xffffffffu, mbar_wait(tmem_empty_bar(buf), bph ^ 1, p.status, kErrMmaWaitTmem, p.launch_tag));
-                RF_STAT_END(w_tmem); }
-                if (!ok) break;
-                { RF_STAT_BEGIN();
-                ok = __all_sync(0xffffffffu, mbar_wait(full_bar(s), ph, p.status, kErrMmaWaitFull, p.launch_tag));
-                RF_STAT_END(w_full); }
-                if (!ok) break;
-                if (TWO) {
+                    { RF_STAT_BEGIN();
+                    ok = mbar_wait(full_bar(s), ph, p.status, kErrMmaWaitFull, p.launch_tag);
+                    RF_STAT_END(w_full); }
+                    if (!ok) break;
+                    tc_fence_after();
                     RF_STAT_BEGIN();
-                    ok = __all_sync(0xffffffffu, mbar_wait(peer_full_bar(s), ph, p.status, kErrMmaWaitFull, p.launch_tag));
-                    RF_STAT_END(w_full);
-                    if (!ok) break;
-                }
-                tc_fence_after();
-                RF_STAT_BEGIN();
-                const uint32_t sa = smem_base + s * Cfg::kStageBytes;
-                const uint64_t adesc = Cfg::kMnMajor ? smem_desc_mnmajor_sw128(sa, BK * 128, 1024)
-                                                     : smem_desc_kmajor_sw128(sa);
-                const uint64_t bdesc = Cfg::kMnMajor ? smem_desc_mnmajor_sw128(sa + Cfg::kABytes, BK * 128, 1024)
-                                                     : smem_desc_kmajor_sw128(sa + Cfg::kABytes);
-                const uint32_t d = tmem_base + buf * BN;
-                if (elect_one()) {
+                    const uint32_t sa = smem_base + s * Cfg::kStageBytes;
+                    const uint64_t adesc = Cfg::kMnMajor ? smem_desc_mnmajor_sw128(sa, BK * 128, 1024)
+                                                         : smem_desc_kmajor_sw128(sa);
+                    const uint64_t bdesc = Cfg::kMnMajor ? smem_desc_mnmajor_sw128(sa + Cfg::kABytes, BK * 128, 1024)
+                                                         : smem_desc_kmajor_sw128(sa + Cfg::kABytes);
+                    const uint32_t d = tmem_base + buf * BN;
 #pragma unroll
-                    for (int j = 0; j < BK / UMMA_K; ++j) {
-                        if (TWO) umma_f8_2cta(d, adesc + kstep * j, bdesc + kstep * j, idesc, j > 0 ? 1u : 0u);
-                        else umma_f8(d, adesc + kstep * j, bdesc + kstep * j, idesc, j > 0 ? 1u : 0u);
-                    }
-                    // One commit per K block (every tcgen05 instruction costs tensor-pipe
-                    // issue time): it publishes the accumulator buffer, and the epilogue,
-                    // which observes it, releases the smem stage on the MMA warp's behalf.
-                    if (TWO) umma_commit_2cta_multicast(tmem_full_bar(buf), 0x3);   // same barrier in both CTAs
-                    else umma_commit(tmem_full_bar(buf));
+                    for (int j = 0; j < BK / UMMA_K; ++j)
+                        umma_f8(d, adesc + kstep * j, bdesc + kstep * j, idesc, j > 0 ? 1u : 0u);
+                    // One commit per K block publishes the accumulator buffer.  128-wide tiles free the smem stage with a
+                    // second one; 256-wide ones leave that to the epilogue, which observes the first (with a second commit,
+                    // and without the arrive in the epilogue's K loop, 6144 x 4608 x 7168 takes 222 us instead of 187: ptxas
+                    // then copies accumulators inside that loop).
+                    umma_commit(tmem_full_bar(buf));
+                    if (Cfg::kCommitFreesStage) umma_commit(empty_bar(s));
+                    RF_STAT_END(w_issue);
                 }
-                __syncwarp();
-                RF_STAT_END(w_issue);
             }
+            RF_STAT_FLUSH(1, w_tmem); RF_STAT_FLUSH(2, w_full); RF_STAT_FLUSH(6, w_issue);
         }
-        if (lane == 0) { RF_STAT_FLUSH(1, w_tmem); RF_STAT_FLUSH(2, w_full); RF_STAT_FLUSH(6, w_issue); }
+        __syncwarp();
     } else if (STREAM_K && warp == 3) {
         // ------------------------------------------------- stream-K flag keeper
         // The fence that publishes this CTA's partial sums and the acquiring polls on other CTAs' flags cost
@@ -526,8 +423,6 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
 #ifdef RF_WAIT_STATS
         const long long t_begin = clock64();
 #endif
-        // (in a CTA pair tmem_empty lives in the leader CTA, the only MMA issuer; both CTAs arrive on it
-        // through the cluster window)
         // K-major scale tables have unit stride along K (a compile-time fact the address arithmetic of the
         // prefetch queue depends on); only the reference's [k/128][m] tables stride by m
         const int as_ks = Cfg::kMnMajor ? (int)p.as_k_stride : 1;
@@ -557,8 +452,7 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
             const TileCoord t = decode_tile(p.splits == 1 ? pc.item : pc.item / p.splits, p.tiles_m, p.tiles_n);
             kb0 = pc.kb0;
             kb1 = pc.kb1;
-            const int cta_m_blk = TWO ? t.m_blk * 2 + (int)cta_rank : t.m_blk;
-            const int row = cta_m_blk * BM + row_in_tile;
+            const int row = t.m_blk * BM + row_in_tile;
             const int col0 = t.n_blk * BN + grp * CPT;
             as_row = p.a_scale + (long long)(row < p.m ? row : 0) * p.as_row_stride;
             bs_row = p.b_scale + (long long)(col0 < p.n ? (col0 >> 7) : 0) * p.bs_row_stride;
@@ -660,16 +554,13 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
                 RF_STAT_END(w_acc); }
                 tc_fence_after();
                 // The MMAs that wrote this buffer have finished reading their smem stage.
-                if (ew == 0 && lane == 0) mbar_arrive(empty_bar(it % STAGES));
+                if (!Cfg::kCommitFreesStage && ew == 0 && lane == 0) mbar_arrive(empty_bar(it % STAGES));
                 const uint32_t taddr = lane_addr + buf * BN + grp * CPT;
                 constexpr int NCH = CPT / 32;
                 auto release_buffer = [&] {
                     tc_fence_before();
                     __syncwarp();
-                    if (lane == 0) {
-                        if (TWO) mbar_arrive_cluster_relaxed(mapa_cluster(tmem_empty_bar(buf), 0));
-                        else mbar_arrive(tmem_empty_bar(buf));
-                    }
+                    if (lane == 0) mbar_arrive(tmem_empty_bar(buf));
                 };
                 RF_STAT_BEGIN();
 #if RF_EPI_WIDE
@@ -761,7 +652,6 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
             {
                 constexpr int SL = Cfg::kSlabs;
                 const TileCoord t = decode_tile(p.splits == 1 ? cur_item : cur_item / p.splits, p.tiles_m, p.tiles_n);
-                const int cta_m_blk = TWO ? t.m_blk * 2 + (int)cta_rank : t.m_blk;
                 const int col0 = t.n_blk * BN + grp * CPT;
                 const uint32_t slab0 = slab_base + ew * SL * Cfg::kSlabBytes;
                 // (128-wide tiles hold 64 accumulators per thread and store one chunk, or two short fp32 ones:
@@ -769,7 +659,7 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
                 constexpr bool kAdvanceMidStore = CPT == 128;
                 constexpr bool kClearInStore = CPT == 128 && SL == 1;
                 bool advanced = false;
-                const int slab_row0 = cta_m_blk * BM + quad * 32;
+                const int slab_row0 = t.m_blk * BM + quad * 32;
                 // One lane hands the slab to the TMA, which clips rows >= m / columns >= n.  Consecutive stores of
                 // this warp alternate over its kSlabs slabs (n_stores counts them across tiles, so skipped chunks
                 // of a ragged tile cannot break the alternation); before a slab is rewritten, the store that last
@@ -904,11 +794,10 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
     // ------------------------------------------------------------- tear-down
     tc_fence_before();
     __syncthreads();
-    if (TWO || CLUSTER_K) cluster_sync_all();     // no other CTA touches this CTA's barriers, smem or TMEM any more
+    if (CLUSTER_K) cluster_sync_all();     // no other CTA touches this CTA's barriers, smem or TMEM any more
     if (warp == 1) {
         tc_fence_after();
-        if (TWO) tmem_dealloc_2cta(tmem_base, Cfg::kTmemCols);
-        else tmem_dealloc(tmem_base, Cfg::kTmemCols);
+        tmem_dealloc(tmem_base, Cfg::kTmemCols);
     }
 }
 
@@ -1000,11 +889,9 @@ fnuz_convert_kernel(const uint4* __restrict__ a, uint4* __restrict__ a_dst, size
 
 using Cfg128 = GemmCfg<128, 6>;
 using Cfg256 = GemmCfg<256, 4>;
-using Cfg256ShortK = GemmCfg<256, 3, false, false, 2>;     // K <= 512: tiles of at most four K blocks
-using CfgPair = GemmCfg<256, 6, true>;      // 256 x 256 tile per CTA pair
-using CfgPair128 = GemmCfg<128, 8, true>;   // 256 x 128 tile per CTA pair: four accumulator buffers in TMEM
-using Cfg128Mn = GemmCfg<128, 6, false, true>;
-using Cfg256Mn = GemmCfg<256, 4, false, true>;
+using Cfg256ShortK = GemmCfg<256, 3, false, 2>;     // K <= 512: tiles of at most four K blocks
+using Cfg128Mn = GemmCfg<128, 6, true>;
+using Cfg256Mn = GemmCfg<256, 4, true>;
 
 // Programmatic dependent launch between consecutive GEMM-path kernels of a stream (the launch latency and
 // the barrier / TMEM set-up of kernel i+1 overlap the tail of kernel i).  RF_FP8_GEMM_PDL=0 switches it off.
@@ -1103,35 +990,18 @@ cudaError_t launch_cfg(const CUtensorMap& tma_a, const CUtensorMap& tma_b, const
         attr_set[dev] = true;
     }
     const int total = p.tiles_m * p.tiles_n * p.splits;
-    if (!Cfg::kTwoCta) {
-        // a stream-K launch shares K blocks out over exactly num_sms CTAs, whatever the tile count
-        const int grid = (total < num_sms && p.sk_tiles == 0) ? total : num_sms;
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(grid, 1, 1);
-        cfg.blockDim = dim3(Cfg::kThreads, 1, 1);
-        cfg.dynamicSmemBytes = Cfg::kSmemBytes;
-        cfg.stream = stream;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[0].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = overlap_launches() ? 1 : 0;
-        return cudaLaunchKernelEx(&cfg, kernel, tma_a, tma_b, tma_c, tma_p, dests, p);
-    }
-    // CTA pairs: clusters of 2 along x, one pair per work item at most
-    const int pairs = total < num_sms / 2 ? total : num_sms / 2;
+    // a stream-K launch shares K blocks out over exactly num_sms CTAs, whatever the tile count
+    const int grid = (total < num_sms && p.sk_tiles == 0) ? total : num_sms;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(2 * pairs, 1, 1);
+    cfg.gridDim = dim3(grid, 1, 1);
     cfg.blockDim = dim3(Cfg::kThreads, 1, 1);
     cfg.dynamicSmemBytes = Cfg::kSmemBytes;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = overlap_launches() ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, tma_a, tma_b, tma_c, tma_p, dests, p);
 }
 
@@ -1209,8 +1079,7 @@ cudaError_t fp8_gemm_prepare_device() {
     if ((e = prepare_cfg<Cfg128, true>()) != cudaSuccess) return e;
     if ((e = prepare_cfg<Cfg256, true>()) != cudaSuccess) return e;
     if ((e = prepare_cfg<Cfg256ShortK>()) != cudaSuccess) return e;
-    if ((e = prepare_cfg<CfgPair>()) != cudaSuccess) return e;
-    if ((e = prepare_cfg<CfgPair128>()) != cudaSuccess) return e;
+    if ((e = fp8_gemm_pair_prepare()) != cudaSuccess) return e;
     if ((e = prepare_cfg<Cfg128Mn>()) != cudaSuccess) return e;
     if ((e = prepare_cfg<Cfg256Mn>()) != cudaSuccess) return e;
     if ((e = prepare_cluster_split<Cfg128>()) != cudaSuccess) return e;
@@ -1249,8 +1118,8 @@ cudaError_t fp8_gemm_launch(const CUtensorMap& tma_a, const CUtensorMap& tma_b, 
     cudaError_t e = mn_major
                         ? (block_n == 256 ? launch_cfg<Cfg256Mn>(tma_a, tma_b, tma_c, tma_p, *dests, p, num_sms, stream)
                                           : launch_cfg<Cfg128Mn>(tma_a, tma_b, tma_c, tma_p, *dests, p, num_sms, stream))
-                    : block_n == 512 ? launch_cfg<CfgPair>(tma_a, tma_b, tma_c, tma_p, *dests, p, num_sms, stream)
-                    : block_n == 384 ? launch_cfg<CfgPair128>(tma_a, tma_b, tma_c, tma_p, *dests, p, num_sms, stream)
+                    : gemm_is_pair(block_n)
+                        ? fp8_gemm_pair_launch(tma_a, tma_b, tma_c, tma_p, *dests, p, block_n, num_sms, overlap_launches(), stream)
                     : block_n == 256
                         ? (short_k_config(p) ? launch_cfg<Cfg256ShortK>(tma_a, tma_b, tma_c, tma_p, *dests, p, num_sms, stream)
                                              : launch_cfg<Cfg256>(tma_a, tma_b, tma_c, tma_p, *dests, p, num_sms, stream))

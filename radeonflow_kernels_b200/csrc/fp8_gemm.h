@@ -51,7 +51,7 @@ struct GemmDestMaps {
 inline bool gemm_is_pair(int block_n) { return block_n == 512 || block_n == 384; }
 inline int gemm_tile_rows(int block_n) { return gemm_is_pair(block_n) ? 256 : 128; }
 inline int gemm_tile_cols(int block_n) { return block_n == 512 ? 256 : (block_n == 384 ? 128 : block_n); }
-inline int gemm_b_box_rows(int block_n) { return block_n == 512 ? 128 : (block_n == 384 ? 64 : block_n); }
+inline int gemm_b_box_rows(int block_n) { return block_n == 512 ? 64 : (block_n == 384 ? 32 : block_n); }
 
 // Scratch a stream-K launch needs: per CTA one fp32 tile slot, then one 64-bit flag per CTA.
 inline size_t gemm_streamk_slot_bytes(int block_n) { return (size_t)128 * gemm_tile_cols(block_n) * sizeof(float); }
@@ -79,6 +79,12 @@ inline int gemm_streamk_tiles(int tiles, int num_sms) {
 cudaError_t fp8_gemm_launch(const CUtensorMap& tma_a, const CUtensorMap& tma_b, const CUtensorMap& tma_c,
                             const CUtensorMap& tma_p, const GemmDestMaps* dests, const GemmParams& p, int block_n,
                             int num_sms, cudaStream_t stream, bool mn_major = false);
+
+// The CTA-pair configurations (fp8_gemm_pair.cu); `overlap`: programmatic dependent launch.
+cudaError_t fp8_gemm_pair_launch(const CUtensorMap& tma_a, const CUtensorMap& tma_b, const CUtensorMap& tma_c,
+                                 const CUtensorMap& tma_p, const GemmDestMaps& dests, const GemmParams& p, int block_n,
+                                 int num_sms, bool overlap, cudaStream_t stream);
+cudaError_t fp8_gemm_pair_prepare();
 
 // The pieces (tile, K slice, first K block, end K block: four ints each) that CTA `unit` of `n_units` works
 // through for launch parameters `p`, in order, computed on the host by the same code the kernel runs (only

@@ -26,15 +26,12 @@ int forced_block_n() {
     return v;
 }
 
-// The CTA-pair configuration (cta_group::2, 256 x 256 per 2-CTA cluster) is correct and selectable
-// (RF_FP8_GEMM_BN=512, or RF_FP8_GEMM_PAIR=1 to let the planner consider it) but is not chosen by
-// default: measured on B200 it runs 6144x4608x7168 at 2.05 PFLOP/s against 2.2 for the one-CTA 128 x 256
-// tile, because the per-K-block accumulator hand-off, not shared-memory bandwidth, bounds both.
+// RF_FP8_GEMM_PAIR=0: the planner never chooses the CTA-pair configuration.
 bool pair_config_enabled() {
     static int v = -1;
     if (v < 0) {
         const char* e = getenv("RF_FP8_GEMM_PAIR");
-        v = (e && atoi(e) == 1) ? 1 : 0;
+        v = (e && e[0] == '0') ? 0 : 1;
     }
     return v == 1;
 }
@@ -133,7 +130,7 @@ GemmPlan plan_for(int m, int n, int k, int num_sms, int bn, int forced_split, co
     return best;
 }
 
-GemmPlan choose_plan_inner(int m, int n, int k, int num_sms, int forced_split, const PlanCosts& c) {
+GemmPlan choose_plan_inner(int m, int n, int k, int num_sms, int forced_split, const PlanCosts& c, bool pairs) {
     const int fb = forced_block_n();
     if (fb) return plan_for(m, n, k, num_sms, fb, forced_split, c);
     // a measured entry for this exact shape beats the model (the caller's explicit split still wins)
@@ -144,34 +141,47 @@ GemmPlan choose_plan_inner(int m, int n, int k, int num_sms, int forced_split, c
     // Wide tiles halve the A traffic and the MMA instruction count per FLOP; prefer them unless
     // they cost noticeably more rounds (ragged N such as 576, or too few tiles).
     GemmPlan best = p256.cost <= p128.cost * 1.02 ? p256 : p128;
-    if (pair_config_enabled()) {
-        GemmPlan pp = plan_for(m, n, k, num_sms, 512, forced_split, c);
-        if (pp.cost < best.cost) best = pp;
+    // One pass of 256-wide tiles that takes at least two rounds runs on CTA pairs, unless their 256 x 256 tiles need a round
+    // more: over 72 such shapes (m 585 .. 8192, us of the pair / the 128 x 256 tile) between 2 % slower and 16 % faster, the
+    // geometric mean 6 %.  In one round the pair's longer hand-offs lose (1337 x 3008 x 1920 11.9 / 11.4; geometric mean of
+    // 169 shapes 20 %), and so does a round more (6232 x 2304 x 2432, 225 pair tiles on 74 pairs, 38.8 / 33.0).
+    const int kb = k / kBlockK;
+    const int tiles = ((m + 127) / 128) * ((n + best.block_n - 1) / best.block_n);
+    const int rounds = (tiles + num_sms - 1) / num_sms;
+    bool pair = false;
+    if (pairs && best.block_n == 256 && best.splits == 1 && rounds > 1) {
+        const int pair_tiles = ((m + 255) / 256) * ((n + 255) / 256);
+        pair = (pair_tiles + num_sms / 2 - 1) / (num_sms / 2) <= rounds;
     }
     // Stream-K instead of a plain single pass, in K blocks of the chosen tile: a plain pass takes
-    // rounds x (kb + per-tile cost), a stream-K pass the even share of all K blocks plus its fixed cost (slot
-    // write, slot read, one more piece per CTA).  Behind whole waves that is about 18 K blocks of a 128 x 256 tile
-    // (7-11 us measured on B200), which pays when a long-K shape has just over a whole number of waves (160 tiles of
-    // 56 K blocks: 2 x 56 against 60.5 + 18); none of the 18 benchmark shapes is such a shape.  With fewer tiles than
-    // SMs every tile has several contributors and a K block takes half the time: about 50 K blocks (256 wide 90;
-    // medians of 154 shapes; 300 x 4160 x 7168 takes 26.6 us, a plain pass 18.1).
-    if (forced_split == 0 && best.splits == 1 && !rf::gemm_is_pair(best.block_n) &&
-        streamk_region(m, n, k, best.block_n, num_sms) > 0) {
-        const int kb = k / kBlockK;
-        const int tiles = ((m + 127) / 128) * ((n + best.block_n - 1) / best.block_n);
-        const int rounds = (tiles + num_sms - 1) / num_sms;
-        const double plain = (double)rounds * (kb + 3.0);
-        const double fixed = rounds > 1 ? 18.0 : (best.block_n == 256 ? 90.0 : 50.0);
+    // rounds x (kb + per-tile cost), 5 % less on pairs, a stream-K pass the even share of all K blocks plus its fixed cost
+    // (slot write, slot read, one more piece per CTA).  Behind whole waves that is about 30 K blocks of a 128 x 256 tile
+    // (us, stream-K / pairs: 887 x 6272 x 6016 42.4 / 44.6, 736 x 7168 x 4352 33.2 / 33.4, 3655 x 2048 x 6144 50.8 / 46.8),
+    // which pays when a long-K shape has just over a whole number of waves (160 tiles of 56 K blocks: 2 x 59 against 66.5 +
+    // 30); none of the 18 benchmark shapes is such a shape.  With fewer tiles than SMs every tile has several contributors
+    // and a K block takes half the time: about 50 K blocks (256 wide 90; medians of 154 shapes; 300 x 4160 x 7168 takes
+    // 26.6 us, a plain pass 18.1).
+    if (forced_split == 0 && best.splits == 1 && streamk_region(m, n, k, best.block_n, num_sms) > 0) {
+        const double plain = (double)rounds * (kb + 3.0) * (pair ? 0.95 : 1.0);
+        const double fixed = rounds > 1 ? 30.0 : (best.block_n == 256 ? 90.0 : 50.0);
         const double shared = (double)tiles * kb / num_sms + 3.0 * (tiles / num_sms + 1) + fixed;
-        if (shared < plain) best.splits = kStreamK;
+        if (shared < plain) {
+            best.splits = kStreamK;
+            pair = false;
+        }
     }
+    if (pair) best.block_n = 512;
     return best;
 }
 
 // forced_split: > 0 = that many K slices, kStreamK = stream-K, 0 = the library's choice.
-GemmPlan choose_plan(int m, int n, int k, int num_sms, int forced_split, bool mn_major = false) {
+// pairs: whether the planner may choose the CTA-pair configuration (it has no stream-K pass and no column-major kernel).
+GemmPlan choose_plan(int m, int n, int k, int num_sms, int forced_split, bool mn_major = false, bool pairs = true) {
     const PlanCosts& costs = mn_major ? kRefLayoutCosts : kRowMajorCosts;
-    GemmPlan plan = choose_plan_inner(m, n, k, num_sms, forced_split == kStreamK ? 1 : forced_split, costs);
+    if (mn_major || forced_split == kStreamK || !pair_config_enabled()) pairs = false;
+    GemmPlan plan = choose_plan_inner(m, n, k, num_sms, forced_split == kStreamK ? 1 : forced_split, costs, pairs);
+    // a table entry of the pair configuration: column-major operands take the one-CTA tiles of its width
+    if (mn_major && plan.block_n == 512 && !forced_block_n()) plan.block_n = 256;
     if (forced_split == kStreamK) plan.splits = kStreamK;
     if (forced_split == 0) {
         const int ov = streamk_override();
@@ -212,7 +222,8 @@ int gemm_impl(const void* a, const void* b, const float* as, const float* bs, vo
     if (split_k > kb) split_k = kb;
     if (split_k > kMaxSplits) split_k = kMaxSplits;
     if (split_k < kStreamK) return RF_ERR_BAD_SHAPE;
-    GemmPlan plan = choose_plan(m, n, k, st->num_sms, split_k, mn_major);
+    // (an N-split GEMM's peer stores were measured from the one-CTA tiles)
+    GemmPlan plan = choose_plan(m, n, k, st->num_sms, split_k, mn_major, n_dest == 1);
     if (mn_major && rf::gemm_is_pair(plan.block_n))
         plan = plan_for(m, n, k, st->num_sms, 256, split_k > 0 ? split_k : 0, kRefLayoutCosts);
     // stream-K serves the row-major single-destination GEMM; elsewhere such a plan runs as a plain pass

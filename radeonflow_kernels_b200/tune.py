@@ -1,6 +1,6 @@
 """Offline tuner of the FP8 GEMM plan table (tile width x split-K or stream-K per shape).
 
-    python -m radeonflow_kernels_b200.tune [--shapes MxNxK,...] [--out plans.txt] [--emit-inc FILE] [--pair]
+    python -m radeonflow_kernels_b200.tune [--shapes MxNxK,...] [--out plans.txt] [--emit-inc FILE] [--no-pair]
 
 The B200 analogue of the reference's brute-force tuner (tuner/gemm_tuner.py:317-549 enumerates kernel
 parameterisations, compiles and times each; tuner/gemm_batch.py:8-27 walks the benchmark shapes) and of
@@ -140,7 +140,8 @@ def main(argv=None):
     ap.add_argument("--shapes", default="", help="MxNxK,... (default: the 18 benchmark shapes)")
     ap.add_argument("--out", default="", help="plan file to write (m n k block_n split_k per line)")
     ap.add_argument("--emit-inc", default="", help="also write the C++ include of the built-in table")
-    ap.add_argument("--pair", action="store_true", help="also time the CTA-pair configuration (block_n 512)")
+    ap.add_argument("--pair", action=argparse.BooleanOptionalAction, default=True,
+                    help="time the CTA-pair configuration (block_n 512) too")
     args = ap.parse_args(argv)
     shapes = parse_shapes(args.shapes) if args.shapes else BENCHMARK_SHAPES
     table = tune(shapes, pair=args.pair)

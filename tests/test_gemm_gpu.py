@@ -297,6 +297,33 @@ def test_library_scratch_and_caller_scratch_give_the_same_bits(rf_lib, m, n, k, 
     assert_close(c1.view(torch.uint16).cpu().numpy(), o.fp8_gemm(a, b, a_s, b_s))
 
 
+@pytest.mark.parametrize("m,n,k,split", [
+    (1, 64, 128, 1), (255, 128, 256, 1), (256, 192, 384, 1), (257, 320, 128, 1), (513, 576, 640, 1),    # edges of one tile
+    (4100, 2368, 640, 1),             # more tiles than pairs: both halves' counters run on over ragged tiles
+    (300, 1088, 1152, 2), (257, 64, 1024, 3), (640, 448, 896, 7)])
+def test_pair_tiles_match_the_oracle_and_the_one_cta_tiles_bits(rf_lib, m, n, k, split):
+    """256 x 256 tiles per CTA pair: row counts around one CTA's 128 and the pair's 256, columns that end in either half,
+    K blocks fewer and more than pipeline stages and scale slots, in one pass and in K slices.  One pass gives the bits of
+    the one-CTA tiles (the same K blocks, promoted in the same order)."""
+    a, b, a_s, b_s = o.generate_input(m, n, k, 17 + m, "randn")
+    da, db, das, dbs = gemm_device_inputs(a, b, a_s, b_s)
+    out = {}
+    try:
+        for bn in (512, 256):
+            assert rf_lib.rf_fp8_gemm_set_plan(m, n, k, bn, split) == 0
+            full, c = canary_output(m, n)
+            for _ in range(2):
+                G.fp8_mm(da, db, das, dbs, c)
+            torch.cuda.synchronize()
+            assert G.device_status() == 0 and canary_intact(full, m, n)
+            out[bn] = c.view(torch.uint16).cpu().numpy()
+    finally:
+        rf_lib.rf_fp8_gemm_set_plan(m, n, k, 0, 0)
+    assert_close(out[512], o.fp8_gemm(a, b, a_s, b_s))
+    if split == 1:
+        assert np.array_equal(out[512], out[256])
+
+
 @pytest.mark.parametrize("block_n", ["512", "384"])
 def test_cta_pair_configuration_matches_oracle(block_n):
     """The cta_group::2 configurations (256 x 256 and 256 x 128 tiles per 2-CTA cluster) are selected per

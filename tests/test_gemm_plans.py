@@ -73,6 +73,25 @@ def test_plan_of_shapes_where_the_costs_are_close(rf_lib, m, n, k, plan):
     assert _get(rf_lib, m, n, k) == plan
 
 
+@pytest.mark.parametrize("m,n,k,plan", [
+    (6000, 4608, 7168, (512, 1)),    # several rounds of wide tiles: CTA pairs
+    (1619, 4096, 1792, (512, 1)),    # two rounds, also of pairs
+    (6232, 2304, 2432, (256, 1)),    # 225 pair tiles on 74 pairs: a round more than the wide tiles need
+    (1337, 3008, 1920, (256, 1)),    # one round
+    (1280, 4096, 7168, (256, tune.STREAM_K)),     # just over one round, long K
+    (3655, 2048, 6144, (512, 1)),    # 1.6 rounds: the second one of pairs costs less than stream-K's fixed part
+])
+def test_plan_between_wide_tiles_pairs_and_stream_k(rf_lib, m, n, k, plan):
+    assert _get(rf_lib, m, n, k) == plan
+    assert rf_lib.rf_fp8_gemm_workspace_bytes(m, n, k, 1) == 0
+
+
+def test_pair_plan_of_the_table_asks_for_no_scratch_in_either_layout(rf_lib):
+    """The column-major entry, which has no pair kernel, runs such an entry as one pass of 256-wide tiles."""
+    assert _get(rf_lib, 1024, 3072, 1536) == (512, 1)
+    assert rf_lib.rf_fp8_gemm_workspace_bytes(1024, 3072, 1536, 0) == 0
+
+
 @pytest.mark.gpu
 def test_plan_is_the_same_with_and_without_a_device(rf_lib):
     code = "from tests.test_gemm_plans import _plan_list; print(_plan_list())"
