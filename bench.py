@@ -53,8 +53,8 @@ NCU_DRAM_BYTES = [18649344, 6402816, 11740928, 2173440, 16908032, 40669696, 1901
 # same two counters for the largest moe_gemm_kernel launch of the single-GPU MoE layer (fc1 of the routed experts and the
 # shared one)
 MOE_NCU_DRAM_BYTES = 2.99e9
-# kernels of one layer through rf_moe_forward: router, top-k, sort (3), row gather, tile list, fc1, fc2, combine
-MOE_LAYER_LAUNCHES = 10
+# kernels of one layer through rf_moe_forward: router, top-k, sort, row gather, fc1, fc2, combine
+MOE_LAYER_LAUNCHES = 7
 METRIC = "fp8_blockscaled_gemm_tflops"
 UNIT = "TFLOP/s"
 

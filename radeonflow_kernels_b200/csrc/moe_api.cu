@@ -146,9 +146,10 @@ size_t max_tiles(int rows, int n_groups, int n_alt) {
     return (size_t)rows / rf::kMoeTileRows + n_groups + (size_t)n_alt / rf::kMoeTileRows + 2;
 }
 
-bool carve_aux(Aux* a, int rows, int n_groups, int n_alt) {
-    const size_t tile_bytes = align_up(max_tiles(rows, n_groups, n_alt) * sizeof(rf::MoeTile), 256);
-    const size_t sort_bytes = align_up(rf::moe_permute_scratch_bytes(rows, n_groups), 256);
+// n_tokens: of a layer, whose tiles may include the shared expert's and whose pairs are sorted; 0 elsewhere
+bool carve_aux(Aux* a, int rows, int n_groups, int n_tokens) {
+    const size_t tile_bytes = align_up(max_tiles(rows, n_groups, n_tokens) * sizeof(rf::MoeTile), 256);
+    const size_t sort_bytes = n_tokens > 0 ? align_up(rf::moe_topk_counts_bytes(n_tokens, n_groups), 256) : 0;
     char* base = static_cast<char*>(rf::device_scratch(tile_bytes + 256 + sort_bytes, rf::kScratchMoeAux));
     if (!base) return false;
     a->tiles = reinterpret_cast<rf::MoeTile*>(base);
@@ -232,7 +233,7 @@ int build_tiles(const int* offsets_dev, int n_groups, int alt_rows, const Aux& a
 // alt group's, behind the n_groups others.
 int grouped_gemm(int nth, const void* x, int n_rows, const void* const* w_host, const void* const* w2_host, int n_groups,
                  int n_out, int k, void* out, const Aux& aux, DeviceState* st, cudaStream_t stream,
-                 const AltGroup& alt = {}, const RowScatter& scatter = {}) {
+                 const AltGroup& alt = {}, const RowScatter& scatter = {}, bool overlap = false) {
     if (n_rows <= 0 && alt.rows <= 0) return RF_OK;
     // result rows leave as 16-byte stores
     if (((uintptr_t)out | (uintptr_t)alt.out) & 15) return RF_ERR_CUDA;
@@ -264,12 +265,12 @@ int grouped_gemm(int nth, const void* x, int n_rows, const void* const* w_host, 
     p.status = st->status;
     p.launch_tag = rf::next_launch_tag();
     const int ctas = g_grid_limit > 0 && g_grid_limit < st->num_sms ? g_grid_limit : st->num_sms;
-    return rf::moe_gemm_launch(w2_host != nullptr, mx, ma, p, ctas, stream) == cudaSuccess ? RF_OK : RF_ERR_CUDA;
+    return rf::moe_gemm_launch(w2_host != nullptr, mx, ma, p, ctas, overlap, stream) == cudaSuccess ? RF_OK : RF_ERR_CUDA;
 }
 
 // logits [n_rows, n_out] = x [n_rows, k] . w [n_out, k]^T + bias
 int router_gemm(const void* x, const void* w, const float* bias, int n_rows, int n_out, int k, void* out,
-                DeviceState* st, cudaStream_t stream) {
+                DeviceState* st, cudaStream_t stream, bool overlap = false) {
     CUtensorMap tx, tw, to;
     if (((uintptr_t)w & 15) ||
         !rf::encode_tma_2d(&tx, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, x, (uint64_t)n_rows, (uint64_t)k, (uint64_t)k * 2,
@@ -294,7 +295,7 @@ int router_gemm(const void* x, const void* w, const float* bias, int n_rows, int
     p.status = st->status;
     p.launch_tag = rf::next_launch_tag();
     const int ctas = g_grid_limit > 0 && g_grid_limit < st->num_sms ? g_grid_limit : st->num_sms;
-    return rf::moe_router_launch(tx, tw, to, p, ctas, stream) == cudaSuccess ? RF_OK : RF_ERR_CUDA;
+    return rf::moe_router_launch(tx, tw, to, p, ctas, overlap, stream) == cudaSuccess ? RF_OK : RF_ERR_CUDA;
 }
 
 // `fill_expanded`: the gathered token rows go to expanded_seq_input (the reference's expand_input output, a stage
@@ -327,45 +328,49 @@ int moe_layer(MoEInputRaw* in, bool compute_router, const float* router_bias, cu
     StageTimer tm(metrics, stream);
     const int t_begin = tm.mark();
 
-    // ---- router GEMM (optional), softmax + top-k, counting sort, row gather  -> "moe_misc"
+    // Each kernel of the layer is a programmatic dependent of the one before it (not with stage times, whose events lie in
+    // between): 128 tokens, 32 experts spent 28 us on the starts of ten kernels.
+    const bool overlap = !metrics;
+    // A shared expert as wide as the routed ones joins their launches as one more group: alone, its 16 and 28 column blocks
+    // (d 7168, f 2048) would occupy 22 and 38 % of the 74 CTA pairs while a small batch streams its weights.  With stage
+    // times asked for it runs by itself, so that each of the reference's stages keeps a time of its own; the arithmetic is
+    // the same.
+    const bool merged = fs == f && !metrics;
+
+    // ---- router GEMM (optional), softmax + top-k, counting sort with the row tiles, row gather  -> "moe_misc"
     if (compute_router) {
-        rc = router_gemm(in->input_seq, in->router_weight, router_bias, T, E, d, in->expert_scores, st, stream);
+        rc = router_gemm(in->input_seq, in->router_weight, router_bias, T, E, d, in->expert_scores, st, stream, overlap);
         if (rc != RF_OK) return rc;
     }
     if (rf::moe_topk_launch(in->expert_scores, T, E, K, in->seq_experts_index, in->seq_experts_softmax,
-                            in->source_rows, stream) != cudaSuccess)
+                            in->source_rows, aux.sort_scratch, overlap, stream) != cudaSuccess)
         return RF_ERR_CUDA;
-    if (rf::moe_permute_launch(in->seq_experts_index, in->source_rows, in->seq_experts_softmax, TK, E,
+    if (rf::moe_permute_launch(in->seq_experts_index, in->source_rows, in->seq_experts_softmax, T, K, E,
                                in->permuted_experts, in->permuted_rows, in->first_token_offset, in->rev_permuted_rows,
-                               in->expanded_seq_softmax, aux.sort_scratch, stream) != cudaSuccess)
+                               in->expanded_seq_softmax, aux.sort_scratch, true, merged ? T : 0, aux.tiles, aux.counters,
+                               overlap, stream) != cudaSuccess)
         return RF_ERR_CUDA;
     void* rows = fill_expanded ? in->expanded_seq_input : in->expanded_fc2_output;
     if (rf::moe_gather_rows_launch(in->input_seq, static_cast<const int*>(in->permuted_rows), T, TK, d * 2, rows,
-                                   st->num_sms, stream) != cudaSuccess)
+                                   st->num_sms, overlap, stream) != cudaSuccess)
         return RF_ERR_CUDA;
     const int t_misc = tm.mark();
     tm.span(1, t_begin, t_misc, 0.0);
 
-    // ---- experts: fc1 (gate and up in one pass, SwiGLU in the epilogue), fc2.  A shared expert as wide as the routed
-    // ones joins their launches as one more group: alone, its 16 and 28 column blocks (d 7168, f 2048) would occupy 22 and
-    // 38 % of the 74 CTA pairs while a small batch streams its weights.  With stage times asked for it runs by itself, so that each of the reference's
-    // stages keeps a time of its own; the arithmetic is the same.
-    const bool merged = fs == f && !metrics;
-    const int* offsets = static_cast<const int*>(in->first_token_offset);
+    // ---- experts: fc1 (gate and up in one pass, SwiGLU in the epilogue), fc2
     std::vector<const void*> wg(in->expert_weight_gate, in->expert_weight_gate + E),
         wu(in->expert_weight_up, in->expert_weight_up + E), wd(in->expert_weight_down, in->expert_weight_down + E);
     wg.push_back(in->shared_expert_weight_gate);
     wu.push_back(in->shared_expert_weight_up);
     wd.push_back(in->shared_expert_weight_down);
     AltGroup s1{in->input_seq, T, in->shared_fc1_output}, s2{in->shared_fc1_output, T, in->shared_fc2_output};
-    if ((rc = build_tiles(offsets, E, merged ? T : 0, aux, stream)) != RF_OK) return rc;
     rc = grouped_gemm(0, rows, TK, wg.data(), wu.data(), E, f, d, in->expanded_fc1_output, aux, st, stream,
-                      merged ? s1 : AltGroup{});
+                      merged ? s1 : AltGroup{}, RowScatter{}, overlap);
     if (rc != RF_OK) return rc;
     const int t_fc1 = tm.mark();
     tm.span(3, t_misc, t_fc1, 2.0 * TK * (double)f * d * 2);
     rc = grouped_gemm(1, in->expanded_fc1_output, TK, wd.data(), nullptr, E, d, f, in->expanded_fc2_output, aux, st, stream,
-                      merged ? s2 : AltGroup{});
+                      merged ? s2 : AltGroup{}, RowScatter{}, overlap);
     if (rc != RF_OK) return rc;
     const int t_fc2 = tm.mark();
     tm.span(4, t_fc1, t_fc2, 2.0 * TK * (double)f * d);
@@ -387,7 +392,7 @@ int moe_layer(MoEInputRaw* in, bool compute_router, const float* router_bias, cu
     // ---- weighted combine + shared add
     if (rf::moe_combine_launch(in->expanded_fc2_output, in->shared_fc2_output,
                                static_cast<const int*>(in->rev_permuted_rows), in->expanded_seq_softmax, T, K, d * 2,
-                               in->final_output, stream) != cudaSuccess)
+                               in->final_output, overlap, stream) != cudaSuccess)
         return RF_ERR_CUDA;
     const int t_end = tm.mark();
     tm.span(11, t_s2, t_end, 0.0);
@@ -535,7 +540,7 @@ int rf_moe_topk(const void* expert_scores, int n_tokens, int n_experts, int top_
         return RF_ERR_UNSUPPORTED;
     if (n_tokens == 0) return RF_OK;
     return rf::moe_topk_launch(expert_scores, n_tokens, n_experts, top_k, seq_experts_index, seq_experts_softmax,
-                               source_rows, reinterpret_cast<cudaStream_t>(stream)) == cudaSuccess
+                               source_rows, nullptr, false, reinterpret_cast<cudaStream_t>(stream)) == cudaSuccess
                ? RF_OK : RF_ERR_CUDA;
 }
 
@@ -555,9 +560,9 @@ int rf_moe_permute(const void* seq_experts_index, const void* source_rows, const
     if (n_tokens == 0)
         return cudaMemsetAsync(first_token_offset, 0, (n_experts + 1) * sizeof(int), s) == cudaSuccess ? RF_OK
                                                                                                         : RF_ERR_CUDA;
-    return rf::moe_permute_launch(seq_experts_index, source_rows, seq_experts_softmax, n_tokens * top_k, n_experts,
+    return rf::moe_permute_launch(seq_experts_index, source_rows, seq_experts_softmax, n_tokens, top_k, n_experts,
                                   permuted_experts, permuted_rows, first_token_offset, rev_permuted_rows,
-                                  expanded_seq_softmax, scratch, s) == cudaSuccess
+                                  expanded_seq_softmax, scratch, false, 0, nullptr, nullptr, false, s) == cudaSuccess
                ? RF_OK : RF_ERR_CUDA;
 }
 
@@ -568,7 +573,7 @@ int rf_moe_gather_rows(const void* input_seq, const void* permuted_rows, int n_t
     DeviceState* st = rf::device_state();
     if (!st) return RF_ERR_CUDA;
     return rf::moe_gather_rows_launch(input_seq, static_cast<const int*>(permuted_rows), n_tokens, n_rows,
-                                      d_hidden * 2, expanded_seq_input, st->num_sms,
+                                      d_hidden * 2, expanded_seq_input, st->num_sms, false,
                                       reinterpret_cast<cudaStream_t>(stream)) == cudaSuccess
                ? RF_OK : RF_ERR_CUDA;
 }
@@ -633,7 +638,7 @@ int rf_moe_combine(const void* expanded_fc2_output, const void* shared_fc2_outpu
         return RF_ERR_NULL_POINTER;
     if (n_tokens < 0 || top_k < 1 || top_k > 8 || d_hidden <= 0 || d_hidden % 8 != 0) return RF_ERR_BAD_SHAPE;
     return rf::moe_combine_launch(expanded_fc2_output, shared_fc2_output, static_cast<const int*>(rev_permuted_rows),
-                                  expanded_seq_softmax, n_tokens, top_k, d_hidden * 2, final_output,
+                                  expanded_seq_softmax, n_tokens, top_k, d_hidden * 2, final_output, false,
                                   reinterpret_cast<cudaStream_t>(stream)) == cudaSuccess
                ? RF_OK : RF_ERR_CUDA;
 }

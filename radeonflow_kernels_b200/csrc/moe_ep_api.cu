@@ -153,7 +153,7 @@ int rf_moe_ep_create(const RfMoeEpConfig* c, RfMoeEp** out) {
                  o_ew = take(TK * 2), o_prank = take(TK * 4), o_prow = take(TK * 4), o_sb = take(E * 4),
                  o_ro = take((ep->E_loc + 1) * 4), o_so = take(2 * 4), o_sh1 = take(T * ep->fs * 2),
                  o_sh2 = take(T * d * 2), o_h = take(cap * f * 2),
-                 o_sort = take(rf_moe_permute_scratch_bytes((int)TK, E) + 16);
+                 o_sort = take(rf::moe_topk_counts_bytes(c->n_tokens, E) + 16);
     if (cudaMalloc(&ep->local, off) != cudaSuccess) { cudaGetLastError(); release(ep); return RF_ERR_CUDA; }
     char* L = ep->local;
     ep->scores = reinterpret_cast<__half*>(L + o_scores);
@@ -286,10 +286,11 @@ int rf_moe_ep_forward(RfMoeEp* ep, const void* x, void* out, rf_stream_t stream)
     ep->n_marks = 0;
     mark(ep, s);
     if ((rc = rf_moe_router_gemm(x, ep->router_w, ep->router_bias, T, E, d, ep->scores, stream)) != RF_OK) return rc;
-    if ((rc = rf_moe_topk(ep->scores, T, E, K, ep->idx, ep->gate_w, ep->source_rows, stream)) != RF_OK) return rc;
-    if ((rc = rf_moe_permute(ep->idx, ep->source_rows, ep->gate_w, T, E, K, ep->perm_experts, ep->perm_rows, ep->first,
-                             ep->rev, ep->exp_w, ep->sort_scratch, stream)) != RF_OK)
-        return rc;
+    if (rf::moe_topk_launch(ep->scores, T, E, K, ep->idx, ep->gate_w, ep->source_rows,
+                            static_cast<int*>(ep->sort_scratch), true, s) != cudaSuccess ||
+        rf::moe_permute_launch(ep->idx, ep->source_rows, ep->gate_w, T, K, E, ep->perm_experts, ep->perm_rows, ep->first,
+                               ep->rev, ep->exp_w, ep->sort_scratch, true, 0, nullptr, nullptr, true, s) != cudaSuccess)
+        return RF_ERR_CUDA;
     // pair counts per global expert (differences of the sorted order's offsets), all-gathered through peer
     // memory; the rendezvous also orders this step after every rank's previous combine
     if ((rc = rendezvous(ep, ep->first, s)) != RF_OK) return rc;

@@ -113,6 +113,7 @@ moe_gemm_kernel(const __grid_constant__ MoeRowMaps x, const __grid_constant__ Mo
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
+    griddep_launch_dependents();
     const int rank = (int)cluster_ctarank();       // 0 = leader of the pair
     const int unit = (int)(blockIdx.x >> 1);
     const int n_units = (int)(gridDim.x >> 1);
@@ -139,6 +140,8 @@ moe_gemm_kernel(const __grid_constant__ MoeRowMaps x, const __grid_constant__ Mo
     cluster_sync_all();      // both CTAs' barriers exist before any remote arrive, byte count or commit
     tc_fence_after();
     const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(tmem_slot_ptr);
+
+    griddep_wait();      // the tile list, the rows and the counters come from the kernels before this one
 
     const int nbn = (p.n_out + TILE_N - 1) / TILE_N;
     const int total_work = __ldg(p.tile_count) * nbn;
@@ -355,7 +358,7 @@ moe_gemm_kernel(const __grid_constant__ MoeRowMaps x, const __grid_constant__ Mo
 }
 
 template <bool SWIGLU>
-cudaError_t launch_mode(const MoeRowMaps& x, const MoeRowMaps& alt, const MoeGemmParams& p, int num_sms,
+cudaError_t launch_mode(const MoeRowMaps& x, const MoeRowMaps& alt, const MoeGemmParams& p, int num_sms, bool overlap,
                         cudaStream_t stream) {
     static bool attr_set[64] = {};
     int dev = 0;
@@ -367,15 +370,24 @@ cudaError_t launch_mode(const MoeRowMaps& x, const MoeRowMaps& alt, const MoeGem
         attr_set[dev] = true;
     }
     const int pairs = num_sms >= 2 ? num_sms / 2 : 1;
-    kernel<<<2 * pairs, THREADS, SMEM_BYTES, stream>>>(x, alt, p);
-    return cudaGetLastError();
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2 * pairs, 1, 1);
+    cfg.blockDim = dim3(THREADS, 1, 1);
+    cfg.dynamicSmemBytes = SMEM_BYTES;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = overlap ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, x, alt, p);
 }
 
 }  // namespace
 
 cudaError_t moe_gemm_launch(bool swiglu, const MoeRowMaps& x, const MoeRowMaps& alt, const MoeGemmParams& p,
-                            int num_sms, cudaStream_t stream) {
-    return swiglu ? launch_mode<true>(x, alt, p, num_sms, stream) : launch_mode<false>(x, alt, p, num_sms, stream);
+                            int num_sms, bool overlap, cudaStream_t stream) {
+    return swiglu ? launch_mode<true>(x, alt, p, num_sms, overlap, stream) : launch_mode<false>(x, alt, p, num_sms, overlap, stream);
 }
 
 }  // namespace rf

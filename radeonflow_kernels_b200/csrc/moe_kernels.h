@@ -6,17 +6,7 @@
 
 namespace rf {
 
-// ---- routing / data movement (moe_route.cu)
-cudaError_t moe_topk_launch(const void* scores, int n_tokens, int n_experts, int top_k, void* index, void* weight,
-                            void* source_rows, cudaStream_t stream);
-size_t moe_permute_scratch_bytes(int n_items, int n_experts);
-cudaError_t moe_permute_launch(const void* experts, const void* source_rows, const void* weights, int n_items,
-                               int n_experts, void* permuted_experts, void* permuted_rows, void* first_token_offset,
-                               void* rev_permuted_rows, void* expanded_softmax, void* scratch, cudaStream_t stream);
-cudaError_t moe_gather_rows_launch(const void* src, const int* row_map, int row_mod, int n_rows, int row_bytes,
-                                   void* dst, int num_sms, cudaStream_t stream);
-cudaError_t moe_combine_launch(const void* y, const void* shared_out, const int* rev, const void* expanded_softmax,
-                               int n_tokens, int top_k, int row_bytes, void* out, cudaStream_t stream);
+// ---- routing / data movement (moe_route.cu); `overlap`: programmatic dependent launch
 // Row ranges [offsets[g], offsets[g + 1]) -> list of row tiles for the grouped GEMM.  With alt_rows > 0 the list
 // starts with the tiles of one more group, number n_groups, of rows [0, alt_rows) of a matrix of its own (the
 // shared expert's).  At most alt_rows / kMoeTileRows + rows / kMoeTileRows + n_groups + 1 tiles.
@@ -28,6 +18,23 @@ struct MoeTile {
 };
 // counters: [0] = number of tiles, [1 .. kMoeItemCounters] = 0, the item counters of as many grouped GEMMs.
 constexpr int kMoeItemCounters = 2;
+
+// block_counts (moe_topk_counts_bytes, or nullptr): the counts that moe_permute_launch needs.
+cudaError_t moe_topk_launch(const void* scores, int n_tokens, int n_experts, int top_k, void* index, void* weight,
+                            void* source_rows, int* block_counts, bool overlap, cudaStream_t stream);
+size_t moe_topk_counts_bytes(int n_tokens, int n_experts);
+size_t moe_permute_scratch_bytes(int n_items, int n_experts);
+// counted: `scratch` holds the counts that moe_topk_launch left for the same tokens; else it has
+// moe_permute_scratch_bytes.  tiles / counters (or nullptr): the
+// row tiles of the experts' rows and of alt_rows rows of an alt group, as moe_tile_list_launch gives them.
+cudaError_t moe_permute_launch(const void* experts, const void* source_rows, const void* weights, int n_tokens, int top_k,
+                               int n_experts, void* permuted_experts, void* permuted_rows, void* first_token_offset,
+                               void* rev_permuted_rows, void* expanded_softmax, void* scratch, bool counted, int alt_rows,
+                               MoeTile* tiles, int* counters, bool overlap, cudaStream_t stream);
+cudaError_t moe_gather_rows_launch(const void* src, const int* row_map, int row_mod, int n_rows, int row_bytes,
+                                   void* dst, int num_sms, bool overlap, cudaStream_t stream);
+cudaError_t moe_combine_launch(const void* y, const void* shared_out, const int* rev, const void* expanded_softmax,
+                               int n_tokens, int top_k, int row_bytes, void* out, bool overlap, cudaStream_t stream);
 cudaError_t moe_tile_list_launch(const int* offsets, int n_groups, int alt_rows, MoeTile* tiles, int* counters,
                                  cudaStream_t stream);
 
@@ -122,7 +129,7 @@ struct MoeGemmParams {
 
 // x: the operand rows; alt: the alt group's rows.  `num_sms` = most CTAs to launch (two per cluster).
 cudaError_t moe_gemm_launch(bool swiglu, const MoeRowMaps& x, const MoeRowMaps& alt, const MoeGemmParams& p,
-                            int num_sms, cudaStream_t stream);
+                            int num_sms, bool overlap, cudaStream_t stream);
 
 // ---- router GEMM (moe_router.cu); tma_w: boxes of n_out rounded up to 16 rows x 64 columns
 // out[r, n] = fp16(X[r,:] . W[n,:] + bias[n]); W is [N, K] row-major (K contiguous), N <= 256
@@ -137,6 +144,6 @@ struct MoeRouterParams {
     int launch_tag;
 };
 cudaError_t moe_router_launch(const CUtensorMap& tma_x, const CUtensorMap& tma_w, const CUtensorMap& tma_out,
-                              const MoeRouterParams& p, int num_sms, cudaStream_t stream);
+                              const MoeRouterParams& p, int num_sms, bool overlap, cudaStream_t stream);
 
 }  // namespace rf

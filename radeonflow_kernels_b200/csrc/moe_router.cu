@@ -5,13 +5,12 @@
 //   warp 1     MMA issuer: 4 x tcgen05.mma.kind::f16 (128 x N x 16) per stage, whole K accumulated in TMEM
 //   warps 4-11 epilogue of the previous tile while the next tile's MMAs run
 //
-// What bounds it: one tile's K loop, at 0.25 to 0.33 us per 64-deep K step.  That depends little on what a step loads or
-// how many steps are in flight (K = 7168, 128 tokens; experts: KB per step, stages, us: 4: 17, 9, 28.6; 32: 20, 9, 31.7;
-// 128: 33, 6, 32.4; 256: 49, 4, 36.8), so it is neither one SM's load rate nor the loads' latency over the stages; which
-// hand-off of a step it is was not taken apart.  N is the experts rounded up to 16, and the stages are as small as that
-// allows and as many as fit: with boxes and MMAs of 256 rows for 32 experts 128 tokens took 42.1 us (now 32.0), 8192
-// tokens 49.0 (36.8).  (K is not split over CTAs: sums in another order round single logits the other way, and a token
-// then chooses another expert.)
+// What bounds it: one tile's K loop.  Producer and issuer run on one lane each: 128 tokens, K = 7168, operands in L2, us as
+// whole warps that vote and elect at every step / now: 4 experts 28.5 / 19.0, 32 experts 31.3 / 21.9, 256 experts 36.7 /
+// 35.7 (there four MMAs of 128 cycles are the step); 8192 tokens 33.0 / 27.2.  Two K steps per stage change nothing (21.5).
+// N is the experts rounded up to 16, and the stages are as small as that allows and as many as fit: with boxes and MMAs of
+// 256 rows for 32 experts 128 tokens took 42.1 us (32.0 with 20 KB stages).  (K is not split over CTAs: sums in another order
+// round single logits the other way, and a token then chooses another expert.)
 #include "ptx.cuh"
 #include "moe_kernels.h"
 
@@ -51,6 +50,7 @@ moe_router_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
+    griddep_launch_dependents();
 
     if (threadIdx.x == 0) {
         tma_prefetch_desc(&tma_a);
@@ -73,6 +73,8 @@ moe_router_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
     tc_fence_after();
     const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(tmem_slot_ptr);
 
+    griddep_wait();
+
     const int total_work = (p.n_rows + BM - 1) / BM;
     const int k_steps = p.k / BK;
     const int n_mma = (p.n_out + 15) & ~15;
@@ -80,54 +82,53 @@ moe_router_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
     const uint32_t n_stages = min((uint32_t)MAX_STAGES, RING_BYTES / stage_bytes);
 
     if (warp == 0) {
-        // ------------------------------------------------------ TMA producer
-        uint32_t s = 0, ph = 0;       // stage, parity of its use
-        bool ok = true;
-        for (int w = blockIdx.x; w < total_work && ok; w += gridDim.x) {
-            const int row0 = w * BM;
-            for (int ks = 0; ks < k_steps; ++ks) {
-                ok = __all_sync(0xffffffffu, mbar_wait(empty_bar(s), ph ^ 1, p.status, kErrProducerWait, p.launch_tag));
-                if (!ok) break;
-                if (elect_one()) {
+        // ------------------------------------------------------ TMA producer (one lane, like the issuer)
+        if (elect_one()) {
+            uint32_t s = 0, ph = 0;       // stage, parity of its use
+            bool ok = true;
+            for (int w = blockIdx.x; w < total_work && ok; w += gridDim.x) {
+                const int row0 = w * BM;
+                for (int ks = 0; ks < k_steps; ++ks) {
+                    ok = mbar_wait(empty_bar(s), ph ^ 1, p.status, kErrProducerWait, p.launch_tag);
+                    if (!ok) break;
                     mbar_expect_tx(full_bar(s), stage_bytes);
                     const uint32_t sa = smem_base + s * stage_bytes;
                     tma_load_2d(sa, &tma_a, full_bar(s), ks * BK, row0);
                     tma_load_2d(sa + A_BYTES, &tma_b, full_bar(s), ks * BK, 0);
+                    if (++s == n_stages) { s = 0; ph ^= 1; }
                 }
-                __syncwarp();
-                if (++s == n_stages) { s = 0; ph ^= 1; }
             }
         }
+        __syncwarp();
     } else if (warp == 1) {
         // -------------------------------------------------------- MMA issuer
-        const uint32_t idesc = make_idesc(BM, n_mma, /*f16*/ 0, /*f16*/ 0, 0, 0);
-        uint32_t s = 0, ph = 0, tcount = 0;
-        bool ok = true;
-        for (int w = blockIdx.x; w < total_work && ok; w += gridDim.x, ++tcount) {
-            const int buf = tcount & 1;
-            const uint32_t bph = (tcount >> 1) & 1;
-            ok = __all_sync(0xffffffffu, mbar_wait(tmem_empty_bar(buf), bph ^ 1, p.status, kErrMmaWaitTmem, p.launch_tag));
-            if (!ok) break;
-            const uint32_t d = tmem_base + buf * BN;
-            for (int ks = 0; ks < k_steps; ++ks) {
-                ok = __all_sync(0xffffffffu, mbar_wait(full_bar(s), ph, p.status, kErrMmaWaitFull, p.launch_tag));
+        if (elect_one()) {
+            const uint32_t idesc = make_idesc(BM, n_mma, /*f16*/ 0, /*f16*/ 0, 0, 0);
+            uint32_t s = 0, ph = 0, tcount = 0;
+            bool ok = true;
+            for (int w = blockIdx.x; w < total_work && ok; w += gridDim.x, ++tcount) {
+                const int buf = tcount & 1;
+                const uint32_t bph = (tcount >> 1) & 1;
+                ok = mbar_wait(tmem_empty_bar(buf), bph ^ 1, p.status, kErrMmaWaitTmem, p.launch_tag);
                 if (!ok) break;
-                tc_fence_after();
-                const uint32_t sa = smem_base + s * stage_bytes;
-                const uint64_t adesc = smem_desc_kmajor_sw128(sa);
-                const uint64_t bdesc = smem_desc_kmajor_sw128(sa + A_BYTES);
-                if (elect_one()) {
+                const uint32_t d = tmem_base + buf * BN;
+                for (int ks = 0; ks < k_steps; ++ks) {
+                    ok = mbar_wait(full_bar(s), ph, p.status, kErrMmaWaitFull, p.launch_tag);
+                    if (!ok) break;
+                    tc_fence_after();
+                    const uint32_t sa = smem_base + s * stage_bytes;
+                    const uint64_t adesc = smem_desc_kmajor_sw128(sa);
+                    const uint64_t bdesc = smem_desc_kmajor_sw128(sa + A_BYTES);
 #pragma unroll
-                    for (int j = 0; j < BK / UMMA_K; ++j) {
+                    for (int j = 0; j < BK / UMMA_K; ++j)
                         umma_f16(d, adesc + 2 * j, bdesc + 2 * j, idesc, (ks > 0 || j > 0) ? 1u : 0u);
-                    }
                     umma_commit(empty_bar(s));
                     if (ks == k_steps - 1) umma_commit(tmem_full_bar(buf));
+                    if (++s == n_stages) { s = 0; ph ^= 1; }
                 }
-                __syncwarp();
-                if (++s == n_stages) { s = 0; ph ^= 1; }
             }
         }
+        __syncwarp();
     } else if (warp >= NUM_NON_EPI_WARPS) {
         // ---------------------------------------------------------- epilogue
         const int ew = warp - NUM_NON_EPI_WARPS;
@@ -223,7 +224,7 @@ moe_router_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
 }  // namespace
 
 cudaError_t moe_router_launch(const CUtensorMap& tma_x, const CUtensorMap& tma_w, const CUtensorMap& tma_out,
-                              const MoeRouterParams& p, int num_sms, cudaStream_t stream) {
+                              const MoeRouterParams& p, int num_sms, bool overlap, cudaStream_t stream) {
     static bool attr_set[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
@@ -234,8 +235,17 @@ cudaError_t moe_router_launch(const CUtensorMap& tma_x, const CUtensorMap& tma_w
         attr_set[dev] = true;
     }
     const int tiles = (p.n_rows + BM - 1) / BM;
-    moe_router_kernel<<<tiles < num_sms ? tiles : num_sms, THREADS, SMEM_BYTES, stream>>>(tma_x, tma_w, tma_out, p);
-    return cudaGetLastError();
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(tiles < num_sms ? tiles : num_sms, 1, 1);
+    cfg.blockDim = dim3(THREADS, 1, 1);
+    cfg.dynamicSmemBytes = SMEM_BYTES;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = overlap ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, moe_router_kernel, tma_x, tma_w, tma_out, p);
 }
 
 }  // namespace rf

@@ -133,6 +133,90 @@ def test_topk_stage_bit_exact(rf_lib, e, k):
     assert np.array_equal(src.cpu().numpy(), rsrc)
 
 
+@pytest.mark.parametrize("e,k", [(4, 2), (32, 8), (256, 8)])
+def test_topk_of_infinite_and_underflowing_logits(rf_lib, e, k):
+    """-inf and logits 80 below the maximum weigh the same; beside a +inf every expert does (exp(-80) each).  Experts whose
+    fp16 probability is zero are chosen by their number."""
+    t = 37
+    rng = np.random.default_rng(e)
+    logits = rng.standard_normal((t, e)).astype(np.float16)
+    finite = logits.copy()
+    logits[:12, 1::2] = -np.inf
+    finite[:12, 1::2] = -60000.0
+    logits[8:16, e // 2] = np.inf
+    finite[8:16] = 0
+    logits[20:24, 0] = finite[20:24, 0] = 200.0            # one expert takes all; the others' probabilities round to zero
+    logits[24] = -np.inf
+    finite[24] = 0
+    d = torch.from_numpy(logits).to(DEV)
+    idx = torch.empty((t, k), dtype=torch.int32, device=DEV)
+    wt = torch.empty((t, k), dtype=torch.float16, device=DEV)
+    src = torch.empty((t * k,), dtype=torch.int32, device=DEV)
+    assert rf_lib.rf_moe_topk(d.data_ptr(), t, e, k, idx.data_ptr(), wt.data_ptr(), src.data_ptr(), None) == 0
+    torch.cuda.synchronize()
+    ridx, rw, rsrc = o.route(finite, k)
+    assert np.array_equal(idx.cpu().numpy(), ridx)
+    assert np.array_equal(wt.cpu().numpy().view(np.uint16), rw.view(np.uint16))
+    assert np.array_equal(src.cpu().numpy(), rsrc)
+
+
+@pytest.mark.parametrize("t,e,k", [(1, 2, 1), (7, 256, 8), (8, 1, 1), (33, 4, 4), (2048, 64, 6), (2049, 32, 3), (2600, 256, 8)])
+def test_routing_of_a_layer_at_the_edges_of_its_sort_blocks(t, e, k):
+    """Top-k's counts, the sort and the row tiles of a layer: a block of 8 tokens and up to 256 blocks, then more tokens a
+    block; few and many counts to add up; one and many experts."""
+    x, w, cfg = o.generate_input(64, 64, e, 1, k, t, 100 + t)
+    rng = np.random.default_rng(t)
+    logits = (rng.standard_normal((t, e)) + 2.0 * rng.standard_normal((1, e))).astype(np.float16)      # a skewed load
+    _, got = run_layer(x, w, cfg, logits=logits)
+    compare_stages(got, o.moe_stages(x[0], w, e, k, logits16=logits))
+
+
+@pytest.mark.parametrize("t,e,k", [(1, 1, 1), (5, 3, 2), (700, 100, 4), (300, 1000, 8), (131073, 24, 2)])
+def test_permute_stage_of_any_expert_count(rf_lib, t, e, k):
+    rng = np.random.default_rng(e)
+    idx = rng.integers(0, e, (t, k)).astype(np.int32)
+    w = rng.random((t, k)).astype(np.float16)
+    src = (np.arange(k, dtype=np.int32)[None, :] * t + np.arange(t, dtype=np.int32)[:, None]).reshape(-1)
+    n = t * k
+    d_idx, d_src, d_w = (torch.from_numpy(a).to(DEV) for a in (idx, src, w))
+    pe, pr, rev = (torch.empty(n, dtype=torch.int32, device=DEV) for _ in range(3))
+    first = torch.empty(e + 1, dtype=torch.int32, device=DEV)
+    ew = torch.empty(n, dtype=torch.float16, device=DEV)
+    size = rf_lib.rf_moe_permute_scratch_bytes(n, e)
+    scratch = torch.full((size + 64,), 0x5A, dtype=torch.uint8, device=DEV)
+    assert rf_lib.rf_moe_permute(d_idx.data_ptr(), d_src.data_ptr(), d_w.data_ptr(), t, e, k, pe.data_ptr(), pr.data_ptr(),
+                                 first.data_ptr(), rev.data_ptr(), ew.data_ptr(), scratch.data_ptr(), None) == 0
+    torch.cuda.synchronize()
+    assert bool((scratch[size:] == 0x5A).all())
+    for got, ref in zip((pe, pr, first, rev), o.permute(idx, src, e)):
+        assert np.array_equal(got.cpu().numpy(), ref)
+    p = pr.cpu().numpy()
+    assert np.array_equal(ew.cpu().numpy().view(np.uint16), w.reshape(-1)[(p % t) * k + p // t].view(np.uint16))
+
+
+def test_row_tiles_of_long_short_and_empty_groups(rf_lib):
+    """Row tiles dealt out over the threads of a block: more tiles than threads, groups without rows in front, in between
+    and at the end, heights around the tile's."""
+    rows = [0, 0, 1, 255, 0, 256, 257, 300000, 17, 0, 2049, 0]
+    k = n = 64
+    g = torch.Generator(device=DEV).manual_seed(5)
+    x = torch.randn((sum(rows), k), generator=g, device=DEV, dtype=torch.float16)
+    ws = [torch.randn((k, n), generator=g, device=DEV, dtype=torch.float16) / 8 for _ in rows]
+    off = torch.tensor(np.concatenate([[0], np.cumsum(rows)]).astype(np.int32), device=DEV)
+    out = torch.full((sum(rows), n), float("nan"), device=DEV, dtype=torch.float16)
+    ptrs = (ctypes.c_void_p * len(rows))(*[w.data_ptr() for w in ws])
+    assert rf_lib.rf_moe_grouped_gemm(x.data_ptr(), sum(rows), ptrs, None, off.data_ptr(), len(rows), n, k, out.data_ptr(),
+                                      None) == 0
+    torch.cuda.synchronize()
+    assert G.device_status() == 0
+    lo = 0
+    for r, w in zip(rows, ws):
+        ref = x[lo:lo + r].float() @ w.float()
+        # fp32 sums of 64 products of order 1/8 each, rounded to fp16
+        torch.testing.assert_close(out[lo:lo + r].float(), ref, rtol=2e-3, atol=2e-3)
+        lo += r
+
+
 def test_permute_stage_large_and_skewed(rf_lib):
     """262144 pairs over 256 experts with a heavy skew and empty experts (config-4 sized)."""
     t, k, e = 32768, 8, 256
