@@ -76,13 +76,13 @@ __device__ __forceinline__ uint32_t swiglu_pair(uint32_t g, uint32_t u) {
 // the pairs running at the same time share that group's weight column block, and the chunk's token rows stay
 // in L2 across all column blocks.  The chunk of work item w is the chunk of tile w / nbn, because the
 // chunks before it hold exactly (first tile of the chunk) * nbn items.
-__device__ __forceinline__ MoeTile decode_item(int w, const MoeTile* __restrict__ tiles, int nbn, int* nb) {
-    const int info = __ldg(&tiles[w / nbn].chunk);
+__device__ __forceinline__ MoeTile decode_item(int w, const MoeTile* tiles, int nbn, int* nb) {
+    const int info = ld_global_s32(&tiles[w / nbn].chunk);
     const int first = info >> 8;
     const int n = info & 0xff;
     const int r = w - first * nbn;
     *nb = r / n;
-    const int4 t = __ldg(reinterpret_cast<const int4*>(tiles + first + r % n));
+    const int4 t = ld_global_v4_s32(tiles + first + r % n);
     return MoeTile{t.x, t.y, t.z, t.w};
 }
 
@@ -144,7 +144,7 @@ moe_gemm_kernel(const __grid_constant__ MoeRowMaps x, const __grid_constant__ Mo
     griddep_wait();      // the tile list, the rows and the counters come from the kernels before this one
 
     const int nbn = (p.n_out + TILE_N - 1) / TILE_N;
-    const int total_work = __ldg(p.tile_count) * nbn;
+    const int total_work = ld_global_s32(p.tile_count) * nbn;
     const int k_steps = p.k / BK;
     // The j-th item of this pair: the first by its number, the later ones as the leader's producer drew them.
     auto wait_item = [&](uint32_t j) {

@@ -15,6 +15,8 @@
 
 namespace rf {
 
+// Kernels that may start before the one in front of them has finished take what it writes through plain pointers (a load
+// from const __restrict__ memory may be moved in front of griddep_wait()).
 namespace {
 
 // exp(x), x <= 0, as a fixed sequence of fp32 operations with no fused multiply-add, so a CPU
@@ -56,7 +58,7 @@ constexpr int kLeastItems = 1024;
 // 32768 tokens x 256 experts, top-8 take 41 us (80 with ten shuffles a round).
 template <int VPT>
 __global__ void __launch_bounds__(1024)
-topk_kernel(const __half* __restrict__ scores, int n_tokens, int n_experts, int top_k, int tokens_per_block,
+topk_kernel(const __half* scores, int n_tokens, int n_experts, int top_k, int tokens_per_block,
             int* __restrict__ out_index, __half* __restrict__ out_weight, int* __restrict__ source_rows,
             int* __restrict__ block_counts) {
     __shared__ int hist[256];
@@ -239,9 +241,8 @@ __device__ void build_tile_list(const int* offsets, int n_groups, int alt_rows, 
 // `tiles`, the row tiles of the grouped GEMMs (build_tile_list).
 // 32768 tokens x top-8, 256 experts: 26 us (118 in three launches, and 34 for the tiles).
 __global__ void __launch_bounds__(1024)
-sort_scatter_kernel(const int* __restrict__ experts, const int* __restrict__ source_rows,
-                    const __half* __restrict__ weights, int n_items, int n_experts, int items_per_block,
-                    const int* __restrict__ block_counts, int* __restrict__ permuted_experts,
+sort_scatter_kernel(const int* experts, const int* source_rows, const __half* weights, int n_items, int n_experts,
+                    int items_per_block, const int* block_counts, int* __restrict__ permuted_experts,
                     int* __restrict__ permuted_rows, int* __restrict__ rev_permuted_rows,
                     __half* __restrict__ expanded_softmax, int* __restrict__ first_token_offset, int alt_rows,
                     MoeTile* __restrict__ tiles, int* __restrict__ counters) {
@@ -332,8 +333,7 @@ sort_scatter_kernel(const int* __restrict__ experts, const int* __restrict__ sou
 
 // dest row r <- src row (row_map[r] % row_mod); one 16-byte vector per thread-iteration
 __global__ void __launch_bounds__(256)
-gather_rows_kernel(const uint4* __restrict__ src, const int* __restrict__ row_map, int row_mod, int n_rows,
-                   int vec_per_row, uint4* __restrict__ dst) {
+gather_rows_kernel(const uint4* src, const int* row_map, int row_mod, int n_rows, int vec_per_row, uint4* dst) {
     griddep_launch_dependents();
     griddep_wait();
     const size_t total = (size_t)n_rows * vec_per_row;
@@ -341,16 +341,15 @@ gather_rows_kernel(const uint4* __restrict__ src, const int* __restrict__ row_ma
         const int r = (int)(i / vec_per_row);
         const int v = (int)(i - (size_t)r * vec_per_row);
         const int s = row_map[r] % row_mod;
-        dst[i] = __ldg(src + (size_t)s * vec_per_row + v);
+        dst[i] = src[(size_t)s * vec_per_row + v];
     }
 }
 
 // out[t, :] = fp16( sum_i w_i * Y[rev[i*T+t], :] + S[t, :] ), fp32 accumulation in rank order
 template <int MAX_K>
 __global__ void __launch_bounds__(256)
-combine_kernel(const uint4* __restrict__ y, const uint4* __restrict__ shared_out, const int* __restrict__ rev,
-               const __half* __restrict__ expanded_softmax, int n_tokens, int top_k, int vec_per_row,
-               uint4* __restrict__ out) {
+combine_kernel(const uint4* y, const uint4* shared_out, const int* rev, const __half* expanded_softmax, int n_tokens,
+               int top_k, int vec_per_row, uint4* out) {
     griddep_launch_dependents();
     griddep_wait();
     const int t = blockIdx.x;
@@ -370,7 +369,7 @@ combine_kernel(const uint4* __restrict__ y, const uint4* __restrict__ shared_out
         uint4 qv[MAX_K];
 #pragma unroll
         for (int i = 0; i < MAX_K; ++i)
-            if (i < top_k) qv[i] = __ldg(y + (size_t)pos_s[i] * vec_per_row + v);
+            if (i < top_k) qv[i] = y[(size_t)pos_s[i] * vec_per_row + v];
 #pragma unroll
         for (int i = 0; i < MAX_K; ++i) {
             if (i >= top_k) continue;
@@ -384,7 +383,7 @@ combine_kernel(const uint4* __restrict__ y, const uint4* __restrict__ shared_out
                 acc[2 * j + 1] = fmaf(w, f.y, acc[2 * j + 1]);
             }
         }
-        const uint4 sq = __ldg(shared_out + (size_t)t * vec_per_row + v);
+        const uint4 sq = shared_out[(size_t)t * vec_per_row + v];
         const __half2* sh = reinterpret_cast<const __half2*>(&sq);
         uint4 o;
         __half2* oh = reinterpret_cast<__half2*>(&o);

@@ -247,6 +247,40 @@ def test_permute_stage_large_and_skewed(rf_lib):
     assert np.array_equal(ew.cpu().numpy().view(np.uint16), w.reshape(-1)[(pr % t) * k + pr // t].view(np.uint16))
 
 
+@pytest.mark.parametrize("t1,t2", [(16, 16), (48, 200), (300, 30)])
+def test_layers_back_to_back_keep_their_own_routing(t1, t2):
+    """The kernels of a layer start while the ones before them still run, and the layers share row tiles and counters: layers
+    of few and of many row tiles in turn, nothing waited for in between, give what each gives alone."""
+    d, f, e, k = 512, 256, 64, 8
+    layers = []
+    for i, t in enumerate((t1, t2, t1)):
+        x, w, cfg = o.generate_input(d, f, e, 1, k, t, 900 + i)
+        rng = np.random.default_rng(i)
+        logits = rng.standard_normal((t, e)).astype(np.float16)
+        if i == 0:
+            logits[:, 8:] -= 20                            # eight experts take everything: few, high row tiles
+        layers.append((torch.from_numpy(x).to(DEV), to_dev(w), cfg, torch.from_numpy(logits).to(DEV)))
+
+    def run(layer):
+        out, buf = M.moe_forward(layer[0], layer[1], layer[2], expert_scores=layer[3])
+        return out, buf.stages["expanded_fc2_output"]
+
+    alone = []
+    for layer in layers:
+        torch.cuda.synchronize()
+        run(layer)
+        torch.cuda.synchronize()
+        alone.append([v.clone() for v in run(layer)])
+        torch.cuda.synchronize()
+    for _ in range(8):
+        got = [run(layers[i % 3]) for i in range(12)]
+        torch.cuda.synchronize()
+        for i, pair in enumerate(got):
+            for v, ref in zip(pair, alone[i % 3]):
+                assert torch.equal(v, ref)
+    assert G.device_status() == 0
+
+
 def test_custom_kernel_matches_moe_forward():
     x, w, cfg = o.generate_input(512, 256, 8, 1, 2, 200, 21)
     tx = torch.from_numpy(x).to(DEV)
