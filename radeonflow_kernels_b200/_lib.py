@@ -94,6 +94,25 @@ def lib() -> ctypes.CDLL:
     return _lib
 
 
+_host = None
+
+
+def host():
+    """The `_host` extension, set up; raises if it has not been built for this interpreter."""
+    global _host
+    if _host is None:
+        import torch
+        try:
+            from . import _host as module
+        except ImportError as e:
+            raise RuntimeError("_host.so is missing or belongs to another interpreter - build it with `python -m "
+                               "radeonflow_kernels_b200.build`") from e
+        module.setup(ctypes.cast(lib().run, ctypes.c_void_p).value, torch._C._cuda_getDevice,
+                     torch._C._cuda_getCurrentRawStream, torch.float8_e4m3fn, torch.float32, torch.bfloat16, torch.float16)
+        _host = module
+    return _host
+
+
 def _declare(L: ctypes.CDLL) -> None:
     vp, ci, sz = ctypes.c_void_p, ctypes.c_int, ctypes.c_size_t
     L.rf_version.restype = ctypes.c_char_p

@@ -1,4 +1,4 @@
-"""In-tree build of librf_b200.so (sm_100a only) with nvcc.
+"""In-tree build of librf_b200.so (sm_100a only) with nvcc, and of the CPython extension _host.so with the host compiler.
 
     python -m radeonflow_kernels_b200.build [--force] [--verbose]
 
@@ -10,10 +10,13 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG_DIR, "csrc")
 LIB_PATH = os.path.join(PKG_DIR, "librf_b200.so")
+HOST_SRC = os.path.join(CSRC, "host_path.cpp")
+HOST_PATH = os.path.join(PKG_DIR, "_host.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -44,7 +47,21 @@ def _stale() -> bool:
     return any(os.path.getmtime(d) > t for d in deps if os.path.exists(d))
 
 
+def build_host(force: bool = False) -> str:
+    """The extension is bound to the interpreter that builds it."""
+    if not force and os.path.exists(HOST_PATH) and os.path.getmtime(HOST_PATH) >= os.path.getmtime(HOST_SRC):
+        return HOST_PATH
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-I" + sysconfig.get_paths()["include"],
+           "-o", HOST_PATH, HOST_SRC]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        sys.stderr.write(res.stdout + res.stderr)
+        raise RuntimeError("building _host.so failed")
+    return HOST_PATH
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
+    build_host(force)
     if not force and not _stale():
         return LIB_PATH
     cmd = [_nvcc()] + NVCC_FLAGS

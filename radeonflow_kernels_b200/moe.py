@@ -51,6 +51,9 @@ def _expert_ptrs(weights, n_experts, j, ctype):
     """
     if n_experts > 0:
         weights[f"experts.{n_experts - 1}.{j}.weight"]      # KeyError before names are made that no weight has
+    packed = (_lib._host or _lib.host()).fp16_addresses(weights, _expert_names(n_experts, j))
+    if packed is not None:
+        return (ctype * n_experts).from_buffer_copy(packed)
     ts = [weights[name] for name in _expert_names(n_experts, j)]
     f16 = torch.float16
     for t in ts:
