@@ -43,13 +43,6 @@ __device__ unsigned long long g_wait_stats[12];
 #define RF_STAT_FLUSH(idx, acc)
 #endif
 
-// RF_EPI_WIDE=1 selects an experimental epilogue inner loop (64 staging registers reloaded in place, the
-// accumulator buffer handed back after two load latencies).  Measured on B200 it is not faster: built without
-// spills it needs the K loop un-unrolled and runs 6144 x 4608 x 7168 in 191 us against 178 us for the default.
-#ifndef RF_EPI_WIDE
-#define RF_EPI_WIDE 0
-#endif
-
 namespace {
 
 constexpr int BM = 128;
@@ -97,9 +90,6 @@ struct GemmCfg {
     static constexpr bool kRebalanceRegs = true;
 #if defined(RF_REGS_LO) && defined(RF_REGS_HI)
     static constexpr int kRegsLo = RF_REGS_LO, kRegsHi = RF_REGS_HI;
-#elif RF_EPI_WIDE
-    static constexpr int kRegsLo = kColsPerThread > 64 ? 40 : 104;
-    static constexpr int kRegsHi = kColsPerThread > 64 ? 232 : 200;
 #else
     static constexpr int kRegsLo = BN == 128 ? 56 : 120, kRegsHi = BN == 128 ? 224 : 192;
 #endif
@@ -439,11 +429,7 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
         // Scale loads run PF K blocks ahead of their use so their latency (L2 or HBM) never sits on the
         // per-K-block critical path.  (Requesting a tile's first scales before the previous tile is stored was
         // measured: no gain on long K, 8 % slower on K <= 512.)
-#if RF_EPI_WIDE
-        constexpr int PF = 3;
-#else
         constexpr int PF = 4;
-#endif
         float qa[PF], qb[PF];
         int kb0 = 0, kb1 = 0;
         const float* as_row = p.a_scale;
@@ -526,17 +512,7 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
                 for (int j = 0; j < CPT / 2; ++j) acc[j] = make_float2(0.f, 0.f);
             }
             zeroed = false;
-#if RF_EPI_WIDE
-            // two 32-column staging buffers, reloaded in place
-            float v[2][32];
-#pragma unroll
-            for (int j = 0; j < 32; ++j) v[0][j] = v[1][j] = 0.f;
-#endif
-#if RF_EPI_WIDE
-#pragma unroll 1
-#else
 #pragma unroll 4
-#endif
             for (int kb = kb0; kb < kb1; ++kb, ++it) {
                 const float s = Cfg::kMnMajor ? qa[0] * qb[0] * out_scale : qa[0] * qb[0];
 #pragma unroll
@@ -563,36 +539,6 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
                     if (lane == 0) mbar_arrive(tmem_empty_bar(buf));
                 };
                 RF_STAT_BEGIN();
-#if RF_EPI_WIDE
-                // The first 64 columns are requested together (two loads: one 64-column load would need 64
-                // consecutive registers, which costs spills); while their FMAs run, the loads of the next two
-                // 32-column chunks are already in flight, so the accumulator buffer is handed back after two
-                // load latencies (one, when the thread owns only 64 columns); the last FMAs run after that.
-                auto fma_chunk = [&](int c, const float (&x)[32]) {
-#pragma unroll
-                    for (int j = 0; j < 16; ++j)
-                        acc[c * 16 + j] = __ffma2_rn(make_float2(x[2 * j], x[2 * j + 1]), s2, acc[c * 16 + j]);
-                };
-                tmem_ld32_async_inplace(taddr, v[0]);
-                tmem_ld32_async_inplace(taddr + 32, v[1]);
-                tmem_ld_fence2(v[0], v[1]);
-                if (NCH == 2) {
-                    release_buffer();
-                    RF_STAT_END(w_rel);
-                    fma_chunk(0, v[0]);
-                    fma_chunk(1, v[1]);
-                } else {
-                    fma_chunk(0, v[0]);
-                    tmem_ld32_async_inplace(taddr + 64, v[0]);
-                    fma_chunk(1, v[1]);
-                    tmem_ld32_async_inplace(taddr + 96, v[1]);
-                    tmem_ld_fence2(v[0], v[1]);
-                    release_buffer();
-                    RF_STAT_END(w_rel);
-                    fma_chunk(2, v[0]);
-                    fma_chunk(3, v[1]);
-                }
-#else
                 // Staging registers: two 32-column buffers (the load of chunk c+1 overlaps the FMAs of
                 // chunk c) when a thread owns 64 columns; one buffer when it owns 128, because 128
                 // accumulators leave no room for a second one (the other epilogue warp on the same
@@ -615,7 +561,6 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
                 }
 #ifdef RF_LATE_RELEASE
                 release_buffer(); RF_STAT_END(w_rel);
-#endif
 #endif
             }
             if (!ok) break;
