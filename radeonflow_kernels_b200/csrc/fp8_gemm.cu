@@ -308,6 +308,7 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
                 }
             }
             RF_STAT_FLUSH(0, w_empty);
+            finish_producer(ok, it, STAGES, empty_bar(0), p.status, kErrProducerWait, p.launch_tag);
         }
         __syncwarp();
     } else if (warp == 1) {

@@ -160,17 +160,8 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_con
                         if (++s == STAGES) { s = 0; ph ^= 1; }
                     }
                 }
-                if (ok) {
-                    // The leader's last commits arrive on this CTA's stage barriers: they have landed before it exits.
-                    for (uint32_t i = 0; i < STAGES && i < it; ++i) {
-                        const uint32_t u = it - 1 - i;
-                        if (!mbar_wait(empty_bar(u % STAGES), (u / STAGES) & 1, p.status, kErrProducerWait, p.launch_tag)) break;
-                    }
-                } else {
-                    // a role gave up: copies in flight land within microseconds; they may not outlive the CTA
-                    const unsigned long long t0 = globaltimer_ns();
-                    while (globaltimer_ns() - t0 < 100000ull) {}
-                }
+                // (the leader's commits arrive on this CTA's stage barriers)
+                finish_producer(ok, it, STAGES, empty_bar(0), p.status, kErrProducerWait, p.launch_tag);
             }
             __syncwarp();
         } else if (warp == 1) {

@@ -203,17 +203,8 @@ moe_gemm_kernel(const __grid_constant__ MoeRowMaps x, const __grid_constant__ Mo
                 w = (int)ld_shared_u32(item_slot(j));
             }
         }
-        if (ok) {
-            // The leader's last commits arrive on this CTA's stage barriers: they have landed before it exits.
-            for (int i = 0; i < STAGES && i < (int)it; ++i) {
-                const uint32_t u = it - 1 - i;
-                if (!mbar_wait(empty_bar(u % STAGES), (u / STAGES) & 1, p.status, kErrProducerWait, p.launch_tag)) break;
-            }
-        } else {
-            // a role gave up: copies in flight land within microseconds; they may not outlive the CTA
-            const unsigned long long t0 = globaltimer_ns();
-            while (globaltimer_ns() - t0 < 100000ull) {}
-        }
+        // (the leader's commits arrive on this CTA's stage barriers)
+        finish_producer(ok, it, STAGES, empty_bar(0), p.status, kErrProducerWait, p.launch_tag);
     } else if (warp == 1 && rank == 0) {
         // -------------------------------------------------------- MMA issuer
         uint32_t it = 0, tcount = 0;

@@ -84,11 +84,11 @@ moe_router_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
     if (warp == 0) {
         // ------------------------------------------------------ TMA producer (one lane, like the issuer)
         if (elect_one()) {
-            uint32_t s = 0, ph = 0;       // stage, parity of its use
+            uint32_t it = 0, s = 0, ph = 0;       // loads so far; stage, parity of its use
             bool ok = true;
             for (int w = blockIdx.x; w < total_work && ok; w += gridDim.x) {
                 const int row0 = w * BM;
-                for (int ks = 0; ks < k_steps; ++ks) {
+                for (int ks = 0; ks < k_steps; ++ks, ++it) {
                     ok = mbar_wait(empty_bar(s), ph ^ 1, p.status, kErrProducerWait, p.launch_tag);
                     if (!ok) break;
                     mbar_expect_tx(full_bar(s), stage_bytes);
@@ -98,6 +98,7 @@ moe_router_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
                     if (++s == n_stages) { s = 0; ph ^= 1; }
                 }
             }
+            finish_producer(ok, it, n_stages, empty_bar(0), p.status, kErrProducerWait, p.launch_tag);
         }
         __syncwarp();
     } else if (warp == 1) {

@@ -129,6 +129,23 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int* st
     }
 }
 
+// End of a TMA producer that has filled `it` stages of a ring of `n_stages`, whose "stage is free" barriers lie at `empty_bar0`,
+// 8 bytes apart.  It waits for the last use of each stage to be over: the tcgen05.commit that frees a stage arrives on its
+// barrier by itself, whenever the MMAs are done, and it has to arrive before the CTA gives its shared memory to another one.
+// That also says that every copy has landed.  Where a role has given up (not `ok`, or one of these waits expires) the copies
+// still in flight land within microseconds; they may not outlive the CTA either.
+__device__ __forceinline__ void finish_producer(bool ok, uint32_t it, uint32_t n_stages, uint32_t empty_bar0, int* status,
+                                                int code, int tag) {
+    for (uint32_t i = 0; ok && i < n_stages && i < it; ++i) {
+        const uint32_t u = it - 1 - i;
+        ok = mbar_wait(empty_bar0 + 8u * (u % n_stages), (u / n_stages) & 1, status, code, tag);
+    }
+    if (!ok) {
+        const unsigned long long t0 = globaltimer_ns();
+        while (globaltimer_ns() - t0 < 100000ull) {}
+    }
+}
+
 // ------------------------------------------------------ flags between CTAs --
 __device__ __forceinline__ void st_release_gpu_u64(unsigned long long* flag, unsigned long long v) {
     asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(flag), "l"(v) : "memory");

@@ -1,0 +1,55 @@
+"""Rules of the kernels that no result shows when they are broken: what they break is an order that the hardware keeps
+nearly always.  Checked on the kernels' source text."""
+import glob
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "radeonflow_kernels_b200", "csrc")
+
+
+def _text(path):
+    """Source without comments."""
+    with open(path) as f:
+        s = f.read()
+    return re.sub(r"//[^\n]*|/\*.*?\*/", "", s, flags=re.S)
+
+
+def _closing(s, start, pair):
+    depth = 0
+    for i in range(start, len(s)):
+        depth += (s[i] == pair[0]) - (s[i] == pair[1])
+        if depth == 0:
+            return i
+    raise AssertionError("unbalanced " + pair)
+
+
+def _kernels():
+    """(file, kernel, parameter list, body) of every kernel."""
+    out = []
+    for path in sorted(glob.glob(os.path.join(CSRC, "*.cu"))):
+        s = _text(path)
+        for m in re.finditer(r"__global__\s+void\s+(?:__\w+__\s*\((?:[^()]|\([^()]*\))*\)\s*)*(\w+)\s*\(", s):
+            end = _closing(s, m.end() - 1, "()")
+            body = s.index("{", end)
+            out.append((os.path.basename(path), m.group(1), s[m.end():end], s[body:_closing(s, body, "{}") + 1]))
+    return out
+
+
+KERNELS = _kernels()
+IDS = [f"{f}:{name}" for f, name, _, _ in KERNELS]
+
+
+def test_every_kernel_is_found():
+    n = sum(len(re.findall(r"__global__", _text(p))) for p in glob.glob(os.path.join(CSRC, "*.cu*")))
+    assert len(KERNELS) == n and n > 10
+
+
+@pytest.mark.parametrize("kernel", KERNELS, ids=IDS)
+def test_commits_on_stage_barriers_are_waited_for(kernel):
+    """A tcgen05.commit that frees a stage arrives on the stage's barrier by itself: the producer waits for the last ones, or
+    they could arrive in shared memory that another CTA has taken over."""
+    _, _, _, body = kernel
+    if re.search(r"umma_commit\w*\(\s*empty_bar", body):
+        assert re.search(r"finish_producer\(\s*ok, it, \w+, empty_bar\(0\)", body)
