@@ -67,9 +67,8 @@ struct PairCfg {
     static constexpr int kChunks = HN_ / 64;                  // 64-column store chunks, one slab each
     static constexpr int kSlabBytes = 32 * 128;
     static constexpr int kStages = HN_ == 128 ? 4 : 6;
-    static constexpr int kScaleSlots = 2 * kBufs;             // K blocks of scale products of each half
-    static constexpr int kScaleBytes = 2 * kScaleSlots * BM * 4;
-    static constexpr int kBarBytes = (2 * kStages + 4 * kBufs) * 8 + 16;
+    static constexpr int kScaleBytes = 2 * kBufs * BM * 4;    // scale products: one slot beside each accumulator buffer
+    static constexpr int kBarBytes = (2 * kStages + 6 * kBufs) * 8 + 16;
     static constexpr int kSmemBytes =
         kStages * kStageBytes + EPI_WARPS * kChunks * kSlabBytes + kScaleBytes + kBarBytes + 1024;
     static_assert(HN_ == 64 || HN_ == 128, "a half holds at most one scale block");
@@ -95,7 +94,8 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_con
     auto empty_bar = [&](uint32_t s) { return bar_base + 8u * (STAGES + s); };
     auto tmem_full_bar = [&](uint32_t b) { return bar_base + 8u * (2 * STAGES + b); };           // b = half * NB + i
     auto tmem_empty_bar = [&](uint32_t b) { return bar_base + 8u * (2 * STAGES + 2 * NB + b); };  // leader's: both CTAs
-    const uint32_t tmem_slot = bar_base + 8u * (2 * STAGES + 4 * NB);
+    auto scale_empty_bar = [&](uint32_t b) { return bar_base + 8u * (2 * STAGES + 4 * NB + b); };
+    const uint32_t tmem_slot = bar_base + 8u * (2 * STAGES + 6 * NB);
     uint32_t* tmem_slot_ptr = reinterpret_cast<uint32_t*>(smem_raw + (tmem_slot - smem_u32(smem_raw)));
 
     const int warp = threadIdx.x >> 5;
@@ -116,6 +116,7 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_con
         for (int b = 0; b < 2 * NB; ++b) {
             mbar_init(tmem_full_bar(b), 2);                // the MMAs' commit and the scale warp
             mbar_init(tmem_empty_bar(b), EPI_WARPS);       // four warps of each CTA
+            mbar_init(scale_empty_bar(b), EPI_WARPS / 2);  // the half's four
         }
         mbar_fence_init();
     }
@@ -205,8 +206,8 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_con
             __syncwarp();
         } else if (warp >= 2) {
             // ------------------------------------------------------ scales
-            // One warp per half: the fp32 products a_s * b_s of this CTA's 128 rows, one K block at a time, into a ring
-            // of slots.  Its loads run PF K blocks ahead, across tiles.
+            // One warp per half: the fp32 products a_s * b_s of this CTA's 128 rows, one K block at a time, into the slot
+            // of the block's accumulator buffer.  Its loads run PF K blocks ahead, across tiles.
             const int half = warp - 2;
             constexpr int PF = 4;
             PlainWalker walk(p, unit, n_units, kb_total);
@@ -243,15 +244,16 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_con
 #pragma unroll
                 for (int d = 0; d < PF; ++d) {
                     if (q >= n_loaded) break;
-                    // A buffer filled for K block q - NB means that the epilogue has given it back after q - 2 NB, whose
-                    // slot this is.
+                    // The epilogue has read the slot for K block q - NB (an order that the hand-back of the accumulator
+                    // does not give: it goes by a relaxed arrive and a commit, which order no shared-memory read).  It
+                    // had then seen that block's arrivals on tmem_full, so this one counts for block q.
                     const uint32_t buf = half * NB + q % NB;
                     if (q >= NB) {
-                        ok = __all_sync(0xffffffffu, mbar_wait(tmem_full_bar(buf), (q / NB - 1) & 1, p.status,
+                        ok = __all_sync(0xffffffffu, mbar_wait(scale_empty_bar(buf), (q / NB - 1) & 1, p.status,
                                                                kErrSchedWait, p.launch_tag));
                         if (!ok) break;
                     }
-                    const uint32_t slot = scale_base + (half * Cfg::kScaleSlots + q % Cfg::kScaleSlots) * (BM * 4);
+                    const uint32_t slot = scale_base + buf * (BM * 4);
                     st_shared_v4(slot + lane * 16, __float_as_uint(qa[d][0] * qb[d]), __float_as_uint(qa[d][1] * qb[d]),
                                  __float_as_uint(qa[d][2] * qb[d]), __float_as_uint(qa[d][3] * qb[d]));
                     __syncwarp();
@@ -269,7 +271,7 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_con
         const int half = ew >> 2;
         const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + half * (NB * HN);
         const uint32_t slab0 = slab_base + ew * Cfg::kChunks * Cfg::kSlabBytes;
-        const uint32_t my_scale = scale_base + half * Cfg::kScaleSlots * (BM * 4) + (quad * 32 + lane) * 4;
+        const uint32_t my_scale = scale_base + half * NB * (BM * 4) + (quad * 32 + lane) * 4;
         PlainWalker walk(p, unit, n_units, kb_total);
         Piece pc;
         uint32_t it = 0;
@@ -289,7 +291,7 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_con
                 const uint32_t taddr = lane_addr + (it % NB) * HN;
                 float v[2][32];
                 tmem_ld32_async(taddr, v[0]);
-                const float s = __uint_as_float(ld_shared_u32(my_scale + (it % Cfg::kScaleSlots) * (BM * 4)));
+                const float s = __uint_as_float(ld_shared_u32(my_scale + (it % NB) * (BM * 4)));
                 const F32x2 s2 = pack_f32x2(s, s);
 #pragma unroll
                 for (int c = 0; c < HN / 32; ++c) {
@@ -298,7 +300,10 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_con
                     if (c + 1 == HN / 32) {
                         tc_fence_before();
                         __syncwarp();
-                        if (lane == 0) mbar_arrive_cluster_relaxed(mapa_cluster(tmem_empty_bar(buf), 0));
+                        if (lane == 0) {
+                            mbar_arrive_cluster_relaxed(mapa_cluster(tmem_empty_bar(buf), 0));
+                            mbar_arrive(scale_empty_bar(buf));
+                        }
                     }
 #pragma unroll
                     for (int j = 0; j < 16; ++j)

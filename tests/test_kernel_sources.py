@@ -53,3 +53,13 @@ def test_commits_on_stage_barriers_are_waited_for(kernel):
     _, _, _, body = kernel
     if re.search(r"umma_commit\w*\(\s*empty_bar", body):
         assert re.search(r"finish_producer\(\s*ok, it, \w+, empty_bar\(0\)", body)
+
+
+def test_a_scale_slot_is_given_back_by_its_readers():
+    """The pair kernel's scale warps rewrite a slot behind a barrier on which the epilogue warps that read it have arrived
+    with release semantics; the accumulator's hand-back (relaxed arrive, commit) orders no shared-memory read."""
+    body = next(b for _, name, _, b in KERNELS if name == "fp8_gemm_pair_kernel")
+    scales, epilogue = body[body.index("warp >= 2"):].split("setmaxnreg.inc", 1)
+    assert scales.index("mbar_wait(scale_empty_bar(buf)") < scales.index("st_shared_v4(slot")
+    assert "tmem_full_bar(buf), (q" not in scales
+    assert epilogue.index("ld_shared_u32(my_scale") < epilogue.index("mbar_arrive(scale_empty_bar(buf))")
