@@ -106,7 +106,7 @@ __device__ __forceinline__ uint32_t fnuz_special(const uint32_t* words) {
     uint32_t v = 0;
 #pragma unroll
     for (int i = 0; i < kFnuzWords / 128; ++i) {
-        const uint4 q = __ldcg(reinterpret_cast<const uint4*>(words) + 32 * i + lane);
+        const uint4 q = ld_global_cg_v4(words + 4 * (32 * i + lane));
         v |= q.x | q.y | q.z | q.w;
     }
     return __reduce_or_sync(0xffffffffu, v);
@@ -446,8 +446,8 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
 #pragma unroll
             for (int d = 0; d < PF; ++d) {
                 const int kk = min(kb0 + d, kb1 - 1);
-                qa[d] = __ldg(as_row + kk * as_ks);
-                qb[d] = __ldg(bs_row + kk * bs_ks);
+                qa[d] = ld_global_f32(as_row + kk * as_ks);
+                qb[d] = ld_global_f32(bs_row + kk * bs_ks);
             }
         };
         // The next piece is drawn (tile decoded, scale pointers set, first scales requested) in the middle of the
@@ -485,7 +485,7 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
                     if (fresh) {
 #pragma unroll
                         for (int q = 0; q < CPT / 4; ++q) {
-                            const float4 t4 = __ldcg(src + q * (32 * Cfg::kEpiWarps));
+                            const float4 t4 = ld_global_cg_v4_f32(src + q * (32 * Cfg::kEpiWarps));
                             acc[2 * q] = make_float2(t4.x, t4.y);
                             acc[2 * q + 1] = make_float2(t4.z, t4.w);
                         }
@@ -495,7 +495,7 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
                         for (int q0 = 0; q0 < CPT / 4; q0 += 8) {
                             float4 t4[8];
 #pragma unroll
-                            for (int i = 0; i < 8; ++i) t4[i] = __ldcg(src + (q0 + i) * (32 * Cfg::kEpiWarps));
+                            for (int i = 0; i < 8; ++i) t4[i] = ld_global_cg_v4_f32(src + (q0 + i) * (32 * Cfg::kEpiWarps));
 #pragma unroll
                             for (int i = 0; i < 8; ++i) {
                                 acc[2 * (q0 + i)].x += t4[i].x;
@@ -520,8 +520,8 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
                 for (int d = 0; d + 1 < PF; ++d) { qa[d] = qa[d + 1]; qb[d] = qb[d + 1]; }
                 {
                     const int kk = min(kb + PF, kb1 - 1);
-                    qa[PF - 1] = __ldg(as_row + kk * as_ks);
-                    qb[PF - 1] = __ldg(bs_row + kk * bs_ks);
+                    qa[PF - 1] = ld_global_f32(as_row + kk * as_ks);
+                    qb[PF - 1] = ld_global_f32(bs_row + kk * bs_ks);
                 }
                 const float2 s2 = make_float2(s, s);
                 const int buf = it % NBUF;
@@ -750,7 +750,7 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
 // C = bf16( sum_s partial[s] )  -  split-K fix-up (reference: reduce_kernel,
 // src/gemm/gemm_kernel.cpp:288-303).  One float4 per thread per slice.
 __global__ void __launch_bounds__(256)
-splitk_reduce_kernel(const float* __restrict__ partial, __nv_bfloat16* __restrict__ c, size_t mn, int splits) {
+splitk_reduce_kernel(const float* partial, __nv_bfloat16* c, size_t mn, int splits) {
     griddep_launch_dependents();
     griddep_wait();     // the slices come from the GEMM launched just before
     const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
@@ -796,8 +796,8 @@ __device__ __forceinline__ uint32_t fnuz_to_fn_x4(uint32_t w, uint32_t& special)
 }
 
 __global__ void __launch_bounds__(kFnuzThreads)
-fnuz_convert_kernel(const uint4* __restrict__ a, uint4* __restrict__ a_dst, size_t a_vec, const uint4* __restrict__ b,
-                    uint4* __restrict__ b_dst, size_t b_vec, uint32_t* __restrict__ words, int* __restrict__ status) {
+fnuz_convert_kernel(const uint4* a, uint4* __restrict__ a_dst, size_t a_vec, const uint4* b, uint4* __restrict__ b_dst,
+                    size_t b_vec, uint32_t* __restrict__ words, int* __restrict__ status) {
     griddep_launch_dependents();
     griddep_wait();       // the GEMM before this call may still be reading the copies and the words
     constexpr int U = 4;  // loads in flight per thread
@@ -808,7 +808,7 @@ fnuz_convert_kernel(const uint4* __restrict__ a, uint4* __restrict__ a_dst, size
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const size_t i = i0 + u * step;
-            if (i < total) q[u] = __ldg(i < a_vec ? a + i : b + (i - a_vec));
+            if (i < total) q[u] = i < a_vec ? a[i] : b[i - a_vec];
         }
 #pragma unroll
         for (int u = 0; u < U; ++u) {

@@ -232,8 +232,8 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_con
             auto load = [&](int d) {
                 if (!more) return;
 #pragma unroll
-                for (int i = 0; i < 4; ++i) qa[d][i] = __ldg(p.a_scale + ar[i]++);
-                qb[d] = __ldg(p.b_scale + br++);
+                for (int i = 0; i < 4; ++i) qa[d][i] = ld_global_f32(p.a_scale + ar[i]++);
+                qb[d] = ld_global_f32(p.b_scale + br++);
                 ++n_loaded;
                 if (--left == 0) more = next_piece();
             };

@@ -324,7 +324,7 @@ moe_gemm_kernel(const __grid_constant__ MoeRowMaps x, const __grid_constant__ Mo
                         if (r < rows_left && col < p.n_out) {
                             __half* row;
                             if (scatter) {
-                                const int meta = __ldg(p.scatter_meta + t.row0 + c0 + r);
+                                const int meta = p.scatter_meta[t.row0 + c0 + r];
                                 row = static_cast<__half*>(pick_peer(p.scatter_dst, meta >> kEpMetaSlotBits)) +
                                       (size_t)(meta & ((1 << kEpMetaSlotBits) - 1)) * p.n_out;
                             } else {

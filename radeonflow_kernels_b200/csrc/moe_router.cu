@@ -167,7 +167,7 @@ moe_router_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
 #pragma unroll
                         for (int j = 0; j < 32; ++j) {
                             const int col = out_col + h * 32 + j;
-                            v[j] += col < p.n_out ? __ldg(p.bias + col) : 0.f;
+                            v[j] += col < p.n_out ? p.bias[col] : 0.f;
                         }
                     }
 #pragma unroll

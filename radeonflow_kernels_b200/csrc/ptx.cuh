@@ -184,8 +184,10 @@ __device__ __forceinline__ void griddep_launch_dependents() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-// What a kernel before this one wrote is read with these behind griddep_wait(), or through plain pointers: a load that the
-// compiler takes for one of constant data (__ldg, const __restrict__) may be moved in front of the wait.
+// What a kernel before this one wrote, or may have written (a caller's operands too), is read behind griddep_wait() with these
+// or through plain pointers: a load that the compiler takes for one of constant data (__ldg, const __restrict__), or for a
+// function of its address alone (__ldcg), may be moved in front of the wait, and the read-only path promises nothing for
+// memory that is written while the kernel runs, which here begins before the kernel in front of it has ended.
 __device__ __forceinline__ int ld_global_s32(const int* p) {
     int v;
     asm volatile("ld.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
@@ -194,6 +196,23 @@ __device__ __forceinline__ int ld_global_s32(const int* p) {
 __device__ __forceinline__ int4 ld_global_v4_s32(const void* p) {
     int4 v;
     asm volatile("ld.global.v4.s32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+    return v;
+}
+
+__device__ __forceinline__ float ld_global_f32(const float* p) {
+    float v;
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+// (past L1: for what other CTAs of this launch write, and what is read once)
+__device__ __forceinline__ uint4 ld_global_cg_v4(const void* p) {
+    uint4 v;
+    asm volatile("ld.global.cg.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ float4 ld_global_cg_v4_f32(const void* p) {
+    float4 v;
+    asm volatile("ld.global.cg.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p) : "memory");
     return v;
 }
 

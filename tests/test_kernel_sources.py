@@ -63,3 +63,24 @@ def test_a_scale_slot_is_given_back_by_its_readers():
     assert scales.index("mbar_wait(scale_empty_bar(buf)") < scales.index("st_shared_v4(slot")
     assert "tmem_full_bar(buf), (q" not in scales
     assert epilogue.index("ld_shared_u32(my_scale") < epilogue.index("mbar_arrive(scale_empty_bar(buf))")
+
+
+def test_dependent_launches_read_nothing_as_constant_data():
+    """A kernel that may start before the one in front of it has finished waits for it and then reads what it wrote: with loads
+    that the compiler cannot move in front of that wait.  (In files with such kernels, the helpers they call included.)"""
+    waiting = [(f, name, params) for f, name, params, body in KERNELS if "griddep_wait()" in body]
+    assert len(waiting) >= 8
+    for f, name, params in waiting:
+        assert not re.search(r"const[^,]*\*\s*__restrict__", params), (f, name)
+    for f in {f for f, _, _ in waiting} | {"ptx.cuh", "fp8_tiles.cuh"}:
+        assert not re.search(r"__ld(g|cg|ca|cs|lu)\(", _text(os.path.join(CSRC, f))), f
+
+
+def test_dependent_launches_wait():
+    """Files that launch kernels as programmatic dependents: each of their kernels waits, or is launched without."""
+    plain = {"sort_count_kernel", "tile_list_kernel"}      # `launch(..., false, ...)`, <<< >>>
+    for f, name, _, body in KERNELS:
+        if "programmaticStreamSerializationAllowed" in _text(os.path.join(CSRC, f)) and name not in plain:
+            assert body.count("griddep_wait()") == 1, (f, name)
+    s = _text(os.path.join(CSRC, "moe_route.cu"))
+    assert re.search(r"launch\(sort_count_kernel, [^;]*?, stream, false,", s) and "tile_list_kernel<<<" in s
