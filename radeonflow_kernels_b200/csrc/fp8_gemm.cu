@@ -264,6 +264,8 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
     // queues behind those of the epilogue warps on the same scheduler.  (1024 x 1536 x 7168 in one pass of 128-wide tiles
     // 18.3 us as whole warps that vote and elect at every step, two of them issuing MMAs in turn; now 17.8.  1024 x 4096 x
     // 512: 6.36, now 6.09.)
+    bool producer = false, loads_ok = true;      // the producer's lane; what it leaves for its end, below
+    uint32_t loads = 0;
     if (warp == 0) {
         // ------------------------------------------------------ TMA producer
         uint32_t it = 0;  // running K-block counter across work items
@@ -308,7 +310,9 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
                 }
             }
             RF_STAT_FLUSH(0, w_empty);
-            finish_producer(ok, it, STAGES, empty_bar(0), p.status, kErrProducerWait, p.launch_tag);
+            producer = true;
+            loads = it;
+            loads_ok = ok;
         }
         __syncwarp();
     } else if (warp == 1) {
@@ -398,6 +402,11 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
         }
     }
     if (CLUSTER_K) cluster_sync_all();     // pairs with the epilogue warps' one in front of the sums
+    // (behind the cluster's barrier, which the sums wait for: in front of it 64 x 576 x 7168 in 8 slices takes 7.59 us, here
+    // 7.29.  In 256-wide tiles, whose stages the epilogue frees, it only makes sure that every copy has landed: 1024 x 4096 x
+    // 512 6.40 us, without it 6.36.)
+    if (producer) finish_producer(loads_ok, loads, STAGES, empty_bar(0), p.status, kErrProducerWait, p.launch_tag);
+    __syncwarp();
     } else {
         // ---------------------------------------------------------- epilogue
         if (Cfg::kRebalanceRegs) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(Cfg::kRegsHi));

@@ -136,6 +136,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int* st
 // still in flight land within microseconds; they may not outlive the CTA either.
 __device__ __forceinline__ void finish_producer(bool ok, uint32_t it, uint32_t n_stages, uint32_t empty_bar0, int* status,
                                                 int code, int tag) {
+#pragma unroll 1
     for (uint32_t i = 0; ok && i < n_stages && i < it; ++i) {
         const uint32_t u = it - 1 - i;
         ok = mbar_wait(empty_bar0 + 8u * (u % n_stages), (u / n_stages) & 1, status, code, tag);

@@ -52,7 +52,7 @@ def test_commits_on_stage_barriers_are_waited_for(kernel):
     they could arrive in shared memory that another CTA has taken over."""
     _, _, _, body = kernel
     if re.search(r"umma_commit\w*\(\s*empty_bar", body):
-        assert re.search(r"finish_producer\(\s*ok, it, \w+, empty_bar\(0\)", body)
+        assert re.search(r"finish_producer\((ok, it|loads_ok, loads), \w+, empty_bar\(0\)", body)
 
 
 def test_a_scale_slot_is_given_back_by_its_readers():
