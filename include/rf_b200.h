@@ -26,7 +26,8 @@ enum {
     RF_OK = 0,
     RF_ERR_BAD_SHAPE = 1,      /* m,n,k violate n%64==0, k%128==0, m>0          */
     RF_ERR_NULL_POINTER = 2,
-    RF_ERR_MISALIGNED = 3,     /* a, b, c must be 16-byte aligned               */
+    RF_ERR_MISALIGNED = 3,     /* an address the kernels cannot take: matrices   */
+                               /* and rows 16 bytes, other arrays their element  */
     RF_ERR_WORKSPACE = 4,      /* caller workspace too small                    */
     RF_ERR_CUDA = 5,           /* a CUDA runtime/driver call failed             */
     RF_ERR_DEVICE_TIMEOUT = 6, /* a bounded device-side wait expired            */

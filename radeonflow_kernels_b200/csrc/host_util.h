@@ -7,6 +7,8 @@
 #include <stddef.h>
 #include <stdint.h>
 
+#include <initializer_list>
+
 #include "status_words.h"
 
 namespace rf {
@@ -33,6 +35,14 @@ enum ScratchSlot {
 // State of the current device; initialises it on first use (allocates the
 // 4-byte status word).  Returns nullptr when a CUDA call fails.
 DeviceState* device_state();
+
+// Whether one of the addresses is no multiple of `align` (a power of two).  The entry points answer RF_ERR_MISALIGNED then: a
+// kernel that moves 16 bytes at a time would lose the context over it.
+inline bool misaligned(std::initializer_list<const void*> ptrs, unsigned align) {
+    uintptr_t bits = 0;
+    for (const void* p : ptrs) bits |= (uintptr_t)p;
+    return (bits & (align - 1)) != 0;
+}
 
 // A fresh tag (1 .. kStatusTagMask) for the next kernel launch that records expired waits.
 int next_launch_tag();

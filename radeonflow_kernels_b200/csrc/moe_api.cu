@@ -320,6 +320,21 @@ int moe_layer(MoEInputRaw* in, bool compute_router, const float* router_bias, cu
     for (const void* ptr : need)
         if (!ptr) return RF_ERR_NULL_POINTER;
     if (compute_router && !in->router_weight) return RF_ERR_NULL_POINTER;
+    // Before anything is enqueued: what is moved 16 bytes at a time (the logits by the top-k of 256 experts and by the router's
+    // tile stores, the weights and rows by the TMA and the row kernels), and the rest by its element.
+    const bool scores16 = compute_router ? E % 64 == 0 : E == 256;
+    if (rf::misaligned({in->input_seq, in->shared_expert_weight_gate, in->shared_expert_weight_up,
+                        in->shared_expert_weight_down, compute_router ? in->router_weight : nullptr,
+                        scores16 ? in->expert_scores : nullptr, fill_expanded ? in->expanded_seq_input : nullptr,
+                        in->expanded_fc1_output, in->expanded_fc2_output, in->shared_fc1_output, in->shared_fc2_output,
+                        in->final_output}, 16) ||
+        rf::misaligned({in->seq_experts_index, in->source_rows, in->permuted_experts, in->permuted_rows,
+                        in->first_token_offset, in->rev_permuted_rows, compute_router ? router_bias : nullptr}, 4) ||
+        rf::misaligned({in->expert_scores, in->seq_experts_softmax, in->expanded_seq_softmax}, 2))
+        return RF_ERR_MISALIGNED;
+    for (int e = 0; e < E; ++e)
+        if (rf::misaligned({in->expert_weight_gate[e], in->expert_weight_up[e], in->expert_weight_down[e]}, 16))
+            return RF_ERR_MISALIGNED;
     DeviceState* st = rf::device_state();
     if (!st) return RF_ERR_CUDA;
     Aux aux;
@@ -539,6 +554,9 @@ int rf_moe_topk(const void* expert_scores, int n_tokens, int n_experts, int top_
     if (n_tokens < 0 || !is_pow2(n_experts) || n_experts > 256 || top_k < 1 || top_k > 8 || top_k > n_experts)
         return RF_ERR_UNSUPPORTED;
     if (n_tokens == 0) return RF_OK;
+    if (rf::misaligned({expert_scores}, n_experts == 256 ? 16 : 2) || rf::misaligned({seq_experts_softmax}, 2) ||
+        rf::misaligned({seq_experts_index, source_rows}, 4))
+        return RF_ERR_MISALIGNED;
     return rf::moe_topk_launch(expert_scores, n_tokens, n_experts, top_k, seq_experts_index, seq_experts_softmax,
                                source_rows, nullptr, false, reinterpret_cast<cudaStream_t>(stream)) == cudaSuccess
                ? RF_OK : RF_ERR_CUDA;
@@ -560,6 +578,10 @@ int rf_moe_permute(const void* seq_experts_index, const void* source_rows, const
     if (n_tokens == 0)
         return cudaMemsetAsync(first_token_offset, 0, (n_experts + 1) * sizeof(int), s) == cudaSuccess ? RF_OK
                                                                                                         : RF_ERR_CUDA;
+    if (rf::misaligned({seq_experts_index, source_rows, permuted_experts, permuted_rows, first_token_offset,
+                        rev_permuted_rows, scratch}, 4) ||
+        rf::misaligned({seq_experts_softmax, expanded_seq_softmax}, 2))
+        return RF_ERR_MISALIGNED;
     return rf::moe_permute_launch(seq_experts_index, source_rows, seq_experts_softmax, n_tokens, top_k, n_experts,
                                   permuted_experts, permuted_rows, first_token_offset, rev_permuted_rows,
                                   expanded_seq_softmax, scratch, false, 0, nullptr, nullptr, false, s) == cudaSuccess
@@ -570,6 +592,8 @@ int rf_moe_gather_rows(const void* input_seq, const void* permuted_rows, int n_t
                        void* expanded_seq_input, rf_stream_t stream) {
     if (!input_seq || !permuted_rows || !expanded_seq_input) return RF_ERR_NULL_POINTER;
     if (d_hidden <= 0 || d_hidden % 8 != 0 || n_tokens <= 0 || n_rows < 0) return RF_ERR_BAD_SHAPE;
+    if (n_rows > 0 && (rf::misaligned({input_seq, expanded_seq_input}, 16) || rf::misaligned({permuted_rows}, 4)))
+        return RF_ERR_MISALIGNED;
     DeviceState* st = rf::device_state();
     if (!st) return RF_ERR_CUDA;
     return rf::moe_gather_rows_launch(input_seq, static_cast<const int*>(permuted_rows), n_tokens, n_rows,
@@ -624,6 +648,11 @@ int rf_moe_router_gemm(const void* x, const void* router_weight, const float* ro
     if (!x || !router_weight || !expert_scores) return RF_ERR_NULL_POINTER;
     if (n_tokens < 0 || n_experts < 1 || n_experts > 256 || d_hidden <= 0 || d_hidden % 64 != 0)
         return RF_ERR_BAD_SHAPE;
+    // (whole 64-column pieces of a row leave as 16-byte stores where every row starts at a multiple of 16 bytes)
+    if (n_tokens > 0 &&
+        (rf::misaligned({x, router_weight}, 16) ||
+         rf::misaligned({expert_scores}, n_experts >= 64 && n_experts % 8 == 0 ? 16 : 2) || rf::misaligned({router_bias}, 4)))
+        return RF_ERR_MISALIGNED;
     DeviceState* st = rf::device_state();
     if (!st) return RF_ERR_CUDA;
     if (n_tokens == 0) return RF_OK;
@@ -637,6 +666,10 @@ int rf_moe_combine(const void* expanded_fc2_output, const void* shared_fc2_outpu
     if (!expanded_fc2_output || !shared_fc2_output || !rev_permuted_rows || !expanded_seq_softmax || !final_output)
         return RF_ERR_NULL_POINTER;
     if (n_tokens < 0 || top_k < 1 || top_k > 8 || d_hidden <= 0 || d_hidden % 8 != 0) return RF_ERR_BAD_SHAPE;
+    if (n_tokens > 0 &&
+        (rf::misaligned({expanded_fc2_output, shared_fc2_output, final_output}, 16) ||
+         rf::misaligned({rev_permuted_rows}, 4) || rf::misaligned({expanded_seq_softmax}, 2)))
+        return RF_ERR_MISALIGNED;
     return rf::moe_combine_launch(expanded_fc2_output, shared_fc2_output, static_cast<const int*>(rev_permuted_rows),
                                   expanded_seq_softmax, n_tokens, top_k, d_hidden * 2, final_output, false,
                                   reinterpret_cast<cudaStream_t>(stream)) == cudaSuccess

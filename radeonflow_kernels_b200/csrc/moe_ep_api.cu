@@ -53,6 +53,7 @@ struct RfMoeEp {
     const float* router_bias = nullptr;
     std::vector<const void*> w_gate, w_up, w_down;
     const void *s_gate = nullptr, *s_up = nullptr, *s_down = nullptr;
+    bool weights_aligned = true;      // all of them as the kernels read them
     cudaStream_t side = nullptr;
     cudaEvent_t ev_ready = nullptr, ev_sent = nullptr;
     // stage timing (optional)
@@ -259,6 +260,10 @@ int rf_moe_ep_set_weights(RfMoeEp* ep, const void* router_weight, const float* r
     ep->s_gate = shared_gate;
     ep->s_up = shared_up;
     ep->s_down = shared_down;
+    ep->weights_aligned =
+        !rf::misaligned({router_weight, shared_gate, shared_up, shared_down}, 16) && !rf::misaligned({router_bias}, 4);
+    for (int j = 0; j < ep->E_loc; ++j)
+        if (rf::misaligned({ep->w_gate[j], ep->w_up[j], ep->w_down[j]}, 16)) ep->weights_aligned = false;
     return RF_OK;
 }
 
@@ -277,6 +282,8 @@ int rf_moe_ep_set_option(RfMoeEp* ep, int option, int value) {
 int rf_moe_ep_forward(RfMoeEp* ep, const void* x, void* out, rf_stream_t stream) {
     if (!ep || !x || !out) return RF_ERR_NULL_POINTER;
     if (!ep->connected || !ep->router_w) return RF_ERR_UNSUPPORTED;
+    // before the first launch: a rank that stopped half-way would keep the others waiting
+    if (rf::misaligned({x, out}, 16) || !ep->weights_aligned) return RF_ERR_MISALIGNED;
     rf::DeviceState* st = rf::device_state();
     if (!st) return RF_ERR_CUDA;
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);

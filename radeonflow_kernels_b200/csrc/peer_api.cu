@@ -45,6 +45,7 @@ int rf_peer_free(void* ptr) {
 int rf_moe_add_rows(void* out, const void* add, int n_rows, int d_hidden, rf_stream_t stream) {
     if (!out || !add) return RF_ERR_NULL_POINTER;
     if (n_rows < 0 || d_hidden <= 0 || d_hidden % 8 != 0) return RF_ERR_BAD_SHAPE;
+    if (n_rows > 0 && rf::misaligned({out, add}, 16)) return RF_ERR_MISALIGNED;
     rf::DeviceState* st = rf::device_state();
     if (!st) return RF_ERR_CUDA;
     return rf::moe_add_rows_launch(out, add, (size_t)n_rows * d_hidden, st->num_sms,
@@ -90,6 +91,9 @@ int rf_moe_ep_dispatch(const void* x, const int* permuted_experts, const int* pe
     if (world < 1 || world > 8 || rank < 0 || rank >= world || n_experts % world != 0 || d_hidden <= 0 ||
         d_hidden % 8 != 0 || n_tokens <= 0 || n_pairs < 0 || capacity < 1)
         return RF_ERR_BAD_SHAPE;
+    if (n_pairs > 0 && (rf::misaligned({x, drop_fill}, 16) ||
+                        rf::misaligned({permuted_experts, permuted_rows, first_token_offset, send_base, pair_rank, pair_row}, 4)))
+        return RF_ERR_MISALIGNED;
     rf::DeviceState* st = rf::device_state();
     if (!st) return RF_ERR_CUDA;
     rf::PeerPtrs pp;
@@ -117,6 +121,10 @@ int rf_moe_ep_combine(void* const* y_all, const void* shared_fc2_output, const i
         return RF_ERR_NULL_POINTER;
     if (world < 1 || world > 8 || top_k < 1 || top_k > 8 || d_hidden <= 0 || d_hidden % 8 != 0 || n_tokens < 0)
         return RF_ERR_BAD_SHAPE;
+    if (n_tokens > 0 &&
+        (rf::misaligned({shared_fc2_output, final_output}, 16) || rf::misaligned({expanded_seq_softmax}, 2) ||
+         rf::misaligned({rev_permuted_rows, pair_rank, pair_row}, 4)))
+        return RF_ERR_MISALIGNED;
     rf::PeerPtrs pp;
     for (int i = 0; i < 8; ++i) pp.p[i] = y_all[i < world ? i : 0];
     for (int i = 0; i < world; ++i)

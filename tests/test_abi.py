@@ -7,6 +7,7 @@ import subprocess
 import sys
 
 import pytest
+import torch
 
 from radeonflow_kernels_b200 import _lib
 
@@ -100,6 +101,89 @@ def test_expert_parallel_entries_validate_on_the_host(rf_lib):
     assert d(x=None) == 2
     assert rf_lib.rf_moe_ep_layout(p16, 0, 3, 8, 64, p16, p16, None) == 1      # 8 experts over 3 ranks
     assert rf_lib.rf_moe_ep_layout(p16, 0, 2, 8, 0, p16, p16, None) == 1       # capacity < 1
+
+
+# (refused before any device work; where there is a GPU, nothing stands behind these addresses)
+no_gpu = pytest.mark.skipif(torch.cuda.is_available(), reason="addresses without memory behind them")
+
+MISALIGNED = 3
+A = 0x7000000                # aligned for everything
+
+# entry -> argument list, {argument position: its alignment}
+STAGE_ENTRIES = {
+    "rf_moe_topk": [([A, 4, 256, 8, A, A, A, None], {0: 16, 4: 4, 5: 2, 6: 4}),
+                    ([A, 4, 128, 8, A, A, A, None], {0: 2})],
+    "rf_moe_permute": [([A, A, A, 4, 32, 4, A, A, A, A, A, A, None],
+                        {0: 4, 1: 4, 2: 2, 6: 4, 7: 4, 8: 4, 9: 4, 10: 2, 11: 4})],
+    "rf_moe_gather_rows": [([A, A, 4, 8, 64, A, None], {0: 16, 1: 4, 5: 16})],
+    "rf_moe_router_gemm": [([A, A, A, 4, 72, 64, A, None], {0: 16, 1: 16, 2: 4, 6: 16}),
+                           ([A, A, A, 4, 32, 64, A, None], {6: 2}), ([A, A, A, 4, 70, 64, A, None], {6: 2})],
+    "rf_moe_combine": [([A, A, A, A, 4, 4, 64, A, None], {0: 16, 1: 16, 2: 4, 3: 2, 7: 16})],
+    "rf_moe_add_rows": [([A, A, 4, 64, None], {0: 16, 1: 16})],
+    "rf_moe_ep_dispatch": [([A, A, A, A, A, 64, 256, 128, 8, 0, 2, 512, (ctypes.c_void_p * 8)(*[A] * 8), None, A, A, A, None],
+                            {0: 16, 1: 4, 2: 4, 3: 4, 4: 4, 14: 4, 15: 4, 16: 16})],
+    "rf_moe_ep_combine": [([(ctypes.c_void_p * 8)(*[A] * 8), A, A, A, A, A, 4, 4, 64, 2, A, None],
+                           {1: 16, 2: 4, 3: 2, 4: 4, 5: 4, 10: 16})],
+}
+
+
+@no_gpu
+@pytest.mark.parametrize("entry", STAGE_ENTRIES)
+def test_moe_stage_entries_refuse_addresses_that_their_kernels_cannot_take(rf_lib, entry):
+    """Half the alignment is refused with a status.  The whole of it is not (the call then fails for want of a device)."""
+    fn = getattr(rf_lib, entry)
+    for args, aligned in STAGE_ENTRIES[entry]:
+        for i, a in aligned.items():
+            bad, good = list(args), list(args)
+            bad[i], good[i] = A + a // 2, A + a
+            assert fn(*bad) == MISALIGNED, (i, a)
+            assert fn(*good) not in (0, MISALIGNED), (i, a)
+
+
+def _layer(n_experts, **fields):
+    """A layer's argument block, every address aligned but those given, and what keeps its arrays alive."""
+    raw = _lib.MoEInputRaw()
+    raw.params = _lib.InputParams(1, 8, 64, 64, n_experts, 2, 1, 0)
+    for name in _lib._MOE_PTR_FIELDS:
+        setattr(raw, name, fields.get(name, A))
+    arrays = {}
+    for name in ("expert_weight_gate", "expert_weight_up", "expert_weight_down"):
+        arrays[name] = (ctypes.c_void_p * n_experts)(*[A] * (n_experts - 1), fields.get(name, A))
+        setattr(raw, name, ctypes.cast(arrays[name], ctypes.POINTER(ctypes.c_void_p)))
+    return raw, arrays
+
+
+@no_gpu
+@pytest.mark.parametrize("field,align", [
+    ("input_seq", 16), ("expert_weight_gate", 16), ("expert_weight_up", 16), ("expert_weight_down", 16),
+    ("shared_expert_weight_gate", 16), ("shared_expert_weight_up", 16), ("shared_expert_weight_down", 16),
+    ("expanded_seq_input", 16), ("expanded_fc1_output", 16), ("expanded_fc2_output", 16), ("shared_fc1_output", 16),
+    ("shared_fc2_output", 16), ("final_output", 16), ("seq_experts_index", 4), ("source_rows", 4), ("permuted_experts", 4),
+    ("permuted_rows", 4), ("first_token_offset", 4), ("rev_permuted_rows", 4), ("seq_experts_softmax", 2),
+    ("expanded_seq_softmax", 2)])
+def test_moe_layer_refuses_misaligned_addresses_before_it_enqueues_anything(rf_lib, field, align):
+    for off, refused in ((align // 2, True), (align, False)):
+        raw, keep = _layer(32, **{field: A + off})
+        for st in (rf_lib.run_topk(ctypes.byref(raw), None, None), rf_lib.rf_moe_forward(ctypes.byref(raw), None, None, None)):
+            assert (st == MISALIGNED) is refused and st != 0
+
+
+@no_gpu
+def test_moe_layer_takes_logits_and_router_as_their_kernels_read_them(rf_lib):
+    def status(fn, n_experts, *bias, **fields):
+        raw, keep = _layer(n_experts, **fields)
+        return fn(ctypes.byref(raw), *bias, None, None)
+    topk, forward = rf_lib.run_topk, rf_lib.rf_moe_forward
+    # logits: 16 bytes at a time with 256 experts, written by tile stores from 64 experts on, else by the element
+    for E, given, computed in ((256, 16, 16), (128, 2, 16), (64, 2, 16), (32, 2, 2)):
+        assert status(topk, E, expert_scores=A + given // 2) == MISALIGNED
+        assert status(topk, E, expert_scores=A + given) != MISALIGNED
+        assert status(forward, E, None, expert_scores=A + computed // 2) == MISALIGNED
+        assert status(forward, E, None, expert_scores=A + computed) != MISALIGNED
+    # the router's weight and bias where it runs
+    assert status(topk, 32, router_weight=A + 8) != MISALIGNED
+    assert status(forward, 32, None, router_weight=A + 8) == MISALIGNED
+    assert status(forward, 32, A + 2) == MISALIGNED and status(forward, 32, A + 4) != MISALIGNED
 
 
 def test_expert_parallel_object_validates_its_configuration(rf_lib):

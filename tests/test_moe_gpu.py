@@ -160,6 +160,23 @@ def test_topk_of_infinite_and_underflowing_logits(rf_lib, e, k):
     assert np.array_equal(src.cpu().numpy(), rsrc)
 
 
+@pytest.mark.parametrize("e,k", [(1, 1), (32, 4), (64, 6), (128, 8)])
+def test_topk_takes_logits_at_any_element(rf_lib, e, k):
+    """Fewer than 256 experts: the logits are read one by one, so they may start at any fp16 element."""
+    t = 70
+    logits = np.random.default_rng(e).standard_normal((t, e)).astype(np.float16)
+    d = torch.zeros(t * e + 1, dtype=torch.float16, device=DEV)
+    d[1:] = torch.from_numpy(logits).to(DEV).view(-1)
+    idx = torch.empty((t, k), dtype=torch.int32, device=DEV)
+    wt = torch.empty((t, k), dtype=torch.float16, device=DEV)
+    src = torch.empty((t * k,), dtype=torch.int32, device=DEV)
+    assert rf_lib.rf_moe_topk(d[1:].data_ptr(), t, e, k, idx.data_ptr(), wt.data_ptr(), src.data_ptr(), None) == 0
+    ridx, rw, rsrc = o.route(logits, k)
+    assert np.array_equal(idx.cpu().numpy(), ridx)
+    assert np.array_equal(wt.cpu().numpy().view(np.uint16), rw.view(np.uint16))
+    assert np.array_equal(src.cpu().numpy(), rsrc)
+
+
 @pytest.mark.parametrize("t,e,k", [(1, 2, 1), (7, 256, 8), (8, 1, 1), (33, 4, 4), (2048, 64, 6), (2049, 32, 3), (2600, 256, 8)])
 def test_routing_of_a_layer_at_the_edges_of_its_sort_blocks(t, e, k):
     """Top-k's counts, the sort and the row tiles of a layer: a block of 8 tokens and up to 256 blocks, then more tokens a
