@@ -1,10 +1,13 @@
 """ctypes binding of librf_b200.so (the C ABI declared in include/rf_b200.h).
 
 There is no fallback: if the shared library is missing or a symbol cannot be
-resolved, importing the binding raises.
+resolved, loading it raises.
 """
 import ctypes
+import importlib.util
 import os
+import sysconfig
+import warnings
 
 PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(PKG_DIR, "librf_b200.so")
@@ -94,21 +97,40 @@ def lib() -> ctypes.CDLL:
     return _lib
 
 
+# the extension is bound to one interpreter, whose tag its name carries
+HOST_PATH = os.path.join(PKG_DIR, "_host" + sysconfig.get_config_var("EXT_SUFFIX"))
 _host = None
 
 
+class _NoHost:
+    """Stands in where there is no extension for this interpreter: every call is left to the Python code, which takes
+    1 to 2 us longer."""
+
+    @staticmethod
+    def gemm(*args):
+        return False
+
+    @staticmethod
+    def fp16_addresses(*args):
+        return None
+
+
 def host():
-    """The `_host` extension, set up; raises if it has not been built for this interpreter."""
+    """The `_host` extension, set up, or its stand-in (with a warning) where it cannot be loaded."""
     global _host
     if _host is None:
         import torch
+        run = ctypes.cast(lib().run, ctypes.c_void_p).value
         try:
-            from . import _host as module
-        except ImportError as e:
-            raise RuntimeError("_host.so is missing or belongs to another interpreter - build it with `python -m "
-                               "radeonflow_kernels_b200.build`") from e
-        module.setup(ctypes.cast(lib().run, ctypes.c_void_p).value, torch._C._cuda_getDevice,
-                     torch._C._cuda_getCurrentRawStream, torch.float8_e4m3fn, torch.float32, torch.bfloat16, torch.float16)
+            spec = importlib.util.spec_from_file_location(__name__.rpartition(".")[0] + "._host", HOST_PATH)
+            module = importlib.util.module_from_spec(spec)
+            spec.loader.exec_module(module)
+            module.setup(run, torch._C._cuda_getDevice, torch._C._cuda_getCurrentRawStream, torch.float8_e4m3fn,
+                         torch.float32, torch.bfloat16, torch.float16)
+        except (ImportError, AttributeError) as e:      # not built for this interpreter; a torch without CUDA
+            warnings.warn(f"{HOST_PATH} cannot be used ({e}): calls take longer on the host; `python -m "
+                          "radeonflow_kernels_b200.build` builds it", RuntimeWarning, stacklevel=2)
+            module = _NoHost
         _host = module
     return _host
 

@@ -1,11 +1,14 @@
 """The native form of the Python boundary (`_host`): what it takes, what it hands back, what it leaves to the Python code.
 On the CPU, with objects that have a tensor's attributes and a stand-in for the library's `run`."""
 import ctypes
+import os
+import sysconfig
+import warnings
 
 import pytest
 import torch
 
-from radeonflow_kernels_b200 import _lib
+from radeonflow_kernels_b200 import _lib, build, gemm, moe
 
 FP8, F32, BF16, F16 = torch.float8_e4m3fn, torch.float32, torch.bfloat16, torch.float16
 
@@ -80,3 +83,60 @@ def test_fp16_addresses(host):
     assert h.fp16_addresses(w, ("a", "c")) is None          # another type
     assert h.fp16_addresses(w, ("a", "d")) is None          # not there
     assert h.fp16_addresses([1], ("a",)) is None
+
+
+def test_the_extension_is_named_after_its_interpreter(rf_lib):
+    """... so that another one does not find it, and building for that one is not skipped as done."""
+    assert build.HOST_PATH == _lib.HOST_PATH and build.HOST_PATH.endswith(sysconfig.get_config_var("EXT_SUFFIX"))
+    assert _lib.host().__file__ == _lib.HOST_PATH and os.path.exists(build.build_host())
+    assert not [f for f in os.listdir(build.PKG_DIR) if f.endswith(".tmp")]
+
+
+@pytest.fixture
+def no_extension(rf_lib, monkeypatch, tmp_path):
+    monkeypatch.setattr(_lib, "_host", None)
+    monkeypatch.setattr(_lib, "HOST_PATH", str(tmp_path / os.path.basename(_lib.HOST_PATH)))
+
+
+def test_without_the_extension_the_python_code_serves_every_call(no_extension):
+    with pytest.warns(RuntimeWarning, match="cannot be used"):
+        assert _lib.host().gemm(*_operands()) is False
+    with warnings.catch_warnings():
+        warnings.simplefilter("error")                      # said once
+        cpu = [torch.zeros(s, dtype=t) for s, t in (((16, 128), FP8), ((64, 128), FP8), ((16, 1), F32), ((1, 1), F32),
+                                                    ((16, 64), BF16))]
+        for call in (gemm.custom_kernel, lambda data: gemm.fp8_mm(*data)):
+            with pytest.raises(ValueError, match="must be CUDA tensors"):
+                call(cpu)
+        w = {f"experts.{i}.1.weight": Fake((4, 4), F16, 0x1000 * (i + 1)) for i in range(3)}
+        assert list(moe._expert_ptrs(w, 3, 1, ctypes.c_ulonglong)) == [0x1000, 0x2000, 0x3000]
+
+
+def test_a_torch_without_cuda_gets_the_python_errors(rf_lib, monkeypatch):
+    monkeypatch.setattr(_lib, "_host", None)
+    monkeypatch.delattr(torch._C, "_cuda_getCurrentRawStream", raising=False)
+    with pytest.warns(RuntimeWarning), pytest.raises(ValueError, match="must be CUDA tensors"):
+        gemm.custom_kernel([torch.zeros(1, 1)] * 5)
+
+
+def test_the_library_is_built_where_the_extension_cannot_be(rf_lib, monkeypatch, capsys):
+    monkeypatch.setenv("CXX", "false")
+    assert build.build_host() == build.HOST_PATH            # there already
+    monkeypatch.setattr(build, "HOST_PATH", build.HOST_PATH + ".other")
+    assert build.build() == build.LIB_PATH and os.path.exists(build.LIB_PATH)
+    assert "without its extension" in capsys.readouterr().err and not os.path.exists(build.HOST_PATH)
+    monkeypatch.setenv("CXX", "no-such-compiler")
+    assert build.build() == build.LIB_PATH
+
+
+@pytest.mark.gpu
+def test_results_without_the_extension_are_the_same_bits(rf_lib, monkeypatch):
+    g = torch.Generator(device="cuda").manual_seed(3)
+    a, b = (torch.randn(s, generator=g, device="cuda").to(FP8) for s in ((96, 256), (192, 256)))
+    a_s, b_s = torch.rand((96, 2), generator=g, device="cuda"), torch.rand((2, 2), generator=g, device="cuda")
+    c = [torch.empty((96, 192), dtype=BF16, device="cuda") for _ in range(2)]
+    assert _lib.host() is not _lib._NoHost
+    gemm.custom_kernel((a, b, a_s, b_s, c[0]))
+    monkeypatch.setattr(_lib, "_host", _lib._NoHost)
+    gemm.custom_kernel((a, b, a_s, b_s, c[1]))
+    assert torch.equal(c[0].view(torch.int16), c[1].view(torch.int16)) and c[0].abs().sum() > 0
