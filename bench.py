@@ -44,12 +44,13 @@ import numpy as np  # noqa: E402
 NK_PAIRS = [(1536, 7168), (3072, 1536), (576, 7168), (7168, 256), (7168, 2048), (4608, 7168), (7168, 2304),
             (512, 7168), (4096, 512)]
 SWEEP = [(m, n, k) for m in (1024, 6144) for (n, k) in NK_PAIRS]
-# dram__bytes_read.sum + dram__bytes_write.sum of fp8_gemm_kernel for each sweep shape, in SWEEP order, from one
+# dram__bytes_read.sum + dram__bytes_write.sum of the GEMM kernel of each sweep shape, in SWEEP order, from one
 # ncu pass (two DRAM counters, --clock-control none, caches flushed before each measured launch) over the fifth
-# sweep of `bench.py --steps 2 --warmup 3 --no-cpu-baseline --no-extras`, taken with the kernel as it is now.
-# Reads = A + B + scales once; C mostly stays in the 126 MB L2 at kernel end, hence traffic < algorithmic.
-NCU_DRAM_BYTES = [18649344, 6402816, 11740928, 2173440, 16908032, 40669696, 19015680, 11283712, 2697984, 57371392,
-                  14570240, 49792255, 30637824, 61002752, 116749312, 66869760, 49148928, 5439488]
+# sweep of `bench.py --steps 2 --warmup 3 --no-cpu-baseline --no-extras`, taken with the kernels as they are now.
+# Reads = A + B + scales once; C mostly stays in the 126 MB L2 at kernel end, hence traffic < algorithmic.  6144 x 4608 x
+# 7168, whose operands and result do not fit the L2 together, reads its operands 1.6 times.
+NCU_DRAM_BYTES = [18649600, 6407424, 11740416, 2171904, 16912640, 40669952, 19018496, 11280896, 2698240,
+                  56980224, 14521856, 49644800, 30270208, 62302976, 155530496, 67401216, 49149696, 5478144]
 # same two counters for the largest moe_gemm_kernel launch of the single-GPU MoE layer (fc1 of the routed experts and the
 # shared one)
 MOE_NCU_DRAM_BYTES = 2.99e9
@@ -599,7 +600,8 @@ def run_extras(args, rank, world, dev, dist, peaks):
         "nvlink_bytes_in_per_gpu": nv_bytes, "roofline_ms": roof_ms, "parity": parity,
         "roofline": {"bound": "tensor" if fl / world / (fp8_peak * 1e12) > nv_bytes / 770e9 else "nvlink",
                      "achieved": roof_ms / ms, "peak": 1.0, "unit": "fraction of the target time", "frac": roof_ms / ms,
-                     "kernel": "fp8_gemm_kernel", "traffic": None,
+                     # (peer stores leave from the one-CTA tiles)
+                     "kernel": "fp8_gemm_pair_kernel" if world == 1 else "fp8_gemm_kernel", "traffic": None,
                      "peak_source": "target time = max(FLOPs per GPU / FP8 peak of this run, C bytes received per GPU "
                                     "/ 770 GB/s measured peer bandwidth)"}}
     cbuf.close()
@@ -905,7 +907,8 @@ def run_gpu_arm(args):
                          "frac_of_2x_bf16_burst": achieved / fp8_assumed,
                          "frac_of_2x_bf16_sustained": achieved / (2.0 * peaks["bf16_tflops_sustained"]),
                          "traffic": (sum(NCU_DRAM_BYTES) / len(NCU_DRAM_BYTES) if not args.shapes else None),
-                         "traffic_note": "DRAM bytes per fp8_gemm_kernel launch, mean over the 18 shapes, from an ncu capture "
+                         "traffic_note": "DRAM bytes per GEMM launch (10 of the 18 shapes run fp8_gemm_pair_kernel, 8 "
+                                         "fp8_gemm_kernel), mean over the 18 shapes, from an ncu capture "
                                          "of one whole sweep after the warm-up sweeps (caches flushed per launch); "
                                          f"algorithmic mean {sum(gemm_bytes(*x) for x in SWEEP) / len(SWEEP):.0f}",
                          "peak_source": ("plain FP8 GEMM of the vendor library (torch._scaled_mm, e4m3 8192^3, best of 10) "
@@ -915,7 +918,7 @@ def run_gpu_arm(args):
                          "hbm_write_only_gbs": round(write_gbs, 1),
                          "hbm_write_only_note": "device memset of 1 GiB measured in this run; the third bound of the "
                                                 "per-shape frac_of_bound_with_write (result bytes / this rate)",
-                         "kernel": "fp8_gemm_kernel"},
+                         "kernel": "fp8_gemm_pair_kernel"},
             "cpu_baseline": cpu,
             "e2e": {"value": e2e_val, "unit": UNIT, "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                     "ms_per_step": e2e_ms},
