@@ -82,8 +82,8 @@ struct GemmCfg {
         STAGES * kStageBytes + kEpiWarps * kSlabs * kSlabBytes + kBarBytes + 1024;       // + alignment slack
     // The epilogue (64 or 128 accumulators per thread plus staging) wants more than the 168 registers a
     // 384-thread CTA starts with, the producer warpgroup far fewer: registers are rebalanced after set-up
-    // (128 * kRegsLo + 256 * kRegsHi <= 64512, the CTA's allocation at 168 per thread).  The splits are measured ones: at
-    // most others ptxas copies accumulators inside the K loop, without a spill to show for it.  256 wide, 6144 x 4608 x
+    // (128 * kRegsLo + 256 * kRegsHi <= 64512, the CTA's allocation at 168 per thread).  The splits are measured ones, each
+    // a build of its own: others are slower without a spill to show for it, for reasons not traced.  256 wide, 6144 x 4608 x
     // 7168: 64 / 216 242 us, 72 / 216 247, 88 / 208 224; 56 / 224, 104 / 200 and 120 / 192 176, of which the last is the
     // fastest of the three on short calls.  128 wide, 68 x 6464 x 3456 in 2 slices: 120 / 192 9.8, no rebalancing 10.1,
     // 56 / 224 9.5.
@@ -355,8 +355,8 @@ fp8_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant
                         umma_f8(d, adesc + kstep * j, bdesc + kstep * j, idesc, j > 0 ? 1u : 0u);
                     // One commit per K block publishes the accumulator buffer.  128-wide tiles free the smem stage with a
                     // second one; 256-wide ones leave that to the epilogue, which observes the first (with a second commit,
-                    // and without the arrive in the epilogue's K loop, 6144 x 4608 x 7168 takes 222 us instead of 187: ptxas
-                    // then copies accumulators inside that loop).
+                    // and without the arrive in the epilogue's K loop, 6144 x 4608 x 7168 takes 222 us instead of 187, with no
+                    // spill to show for it).
                     umma_commit(tmem_full_bar(buf));
                     if (Cfg::kCommitFreesStage) umma_commit(empty_bar(s));
                     RF_STAT_END(w_issue);

@@ -14,12 +14,13 @@
 //   warps 4-11  epilogue, four per half: tcgen05.ld, one FMA per element into 128 (64) register accumulators per thread
 //
 // What bounds it: the power cap on long calls, else the epilogue's K block (barrier, TMEM load, FMAs: about 740 cycles
-// where the tensor cores need 512).  Back to back, us, against the 128 x 256 tile of fp8_gemm.cu on the same box: 6144 x
-// 4608 x 7168 190.9 / 214.9, 6144 x 7168 x 2048 96.0 / 106.3.  On the way there: producer and issuer on one lane each
-// (as whole warps that vote and elect at every step 222 and 113: their instructions queue behind the epilogue's on the
-// shared schedulers); the scale products in warps of their own (loaded by the epilogue threads they cost registers that
-// spill: 230 and 114).  The register split is a measured one: ptxas copies accumulators inside the K loop at most others,
-// without a spill to show for it (64 / 216: 194 and 96, 120 / 192: 277 and 120, 40 / 232: 336 and 154).
+// where the tensor cores need 512).  Calls one after the other through custom_kernel, one box, two runs each, us, against the
+// 128 x 256 tile of fp8_gemm.cu as it is now: 6144 x 4608 x 7168 196.6, 200.3 / 207.9, 207.0; 6144 x 7168 x 2048 102.0,
+// 100.3 / 108.5, 108.7; 16384 x 28672 x 7168 3269, 3265 / 3538, 3535.  On the way there, in short runs on another box that gave
+// 190.9 and 96.0 us for the first two shapes: producer and issuer as whole warps that vote and elect at every step 222 and
+// 113 (their instructions queue behind the epilogue's on the shared schedulers); the scales loaded by the epilogue threads,
+// at the cost of registers that spill, 230 and 114; other register splits, without a spill to show for it and for reasons not
+// traced, 64 / 216 194 and 96, 120 / 192 277 and 120, 40 / 232 336 and 154.
 #include "ptx.cuh"
 #include "fp8_gemm.h"
 #include "fp8_tiles.cuh"
@@ -388,6 +389,11 @@ fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_con
     }
 }
 
+// One pass of 256 x 256 tiles is what the planner chooses.  The other three are there for a caller that asks for them (K
+// slices by a plan entry or argument, 256 x 128 tiles by RF_FP8_GEMM_BN): no shape was found where they are the fastest.
+// us in a graph of launches, the plan / 256 x 256 in 2, 3, 4 slices: 1024 x 1536 x 7168 17.6 / 26.0, 21.7, 29.9; 1024 x 512 x
+// 7168 10.1 / 21.9, 17.5, 16.3; 2048 x 2048 x 4096 20.0 / 33.9, 37.6, 44.6.  256 x 128: 1024 x 7168 x 256 7.7 (the plan 7.8),
+// 6144 x 4096 x 512 21.9 (22.2), 1024 x 1536 x 7168 21.6 (17.6), 6144 x 4608 x 7168 221 (200).
 using Pair256 = PairCfg<128>;     // 256 x 256 tiles
 using Pair128 = PairCfg<64>;      // 256 x 128 tiles
 

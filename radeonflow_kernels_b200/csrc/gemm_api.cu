@@ -104,8 +104,9 @@ GemmPlan plan_for(int m, int n, int k, int num_sms, int bn, int forced_split, co
     const int tiles = ((m + tr - 1) / tr) * ((n + tc - 1) / tc);
     const int kb = k / kBlockK;
     if (rf::gemm_is_pair(bn)) num_sms /= 2;     // work items go to CTA pairs
-    // relative time of one K block of one work item, from in-kernel cycle counts
-    // (128 x 128: ~620 cycles, 128 x 256: ~790, CTA pair 256 x 256: ~925)
+    // relative time of one K block of one work item: 128 x 128 and 128 x 256 from in-kernel cycle counts (~620, ~790).  The
+    // pairs' factors choose the slices where RF_FP8_GEMM_BN asks for pairs; whether a call runs on pairs is decided in rounds
+    // (choose_plan_inner).  Their 256 x 256 tile takes about 850 cycles, the way to the next tile included.
     const double wide = bn == 512 ? 1.5 : (bn == 256 ? 1.25 : (bn == 384 ? 0.8 : 1.0));
     const bool short_pass = kb <= c.short_blocks && ((m + 127) / 128) * ((n + 127) / 128) <= num_sms;
     GemmPlan best{bn, 1, 1e30};
@@ -144,7 +145,9 @@ GemmPlan choose_plan_inner(int m, int n, int k, int num_sms, int forced_split, c
     // One pass of 256-wide tiles that takes at least two rounds runs on CTA pairs, unless their 256 x 256 tiles need a round
     // more: over 72 such shapes (m 585 .. 8192, us of the pair / the 128 x 256 tile) between 2 % slower and 16 % faster, the
     // geometric mean 6 %.  In one round the pair's longer hand-offs lose (1337 x 3008 x 1920 11.9 / 11.4; geometric mean of
-    // 169 shapes 20 %), and so does a round more (6232 x 2304 x 2432, 225 pair tiles on 74 pairs, 38.8 / 33.0).
+    // 169 shapes 20 %), and so does a round more (6232 x 2304 x 2432, 225 pair tiles on 74 pairs, 38.8 / 33.0).  Single
+    // shapes of one round come out even: 1024 x 3072 x 1536, which the table has on pairs, 10.7 to 12.1 / 10.8 one after the
+    // other, 10.5 / 10.6 in a graph.
     const int kb = k / kBlockK;
     const int tiles = ((m + 127) / 128) * ((n + best.block_n - 1) / best.block_n);
     const int rounds = (tiles + num_sms - 1) / num_sms;

@@ -126,7 +126,9 @@ def write_plans(table, path):
 def write_inc(table, path):
     with open(path, "w") as f:
         f.write("// {m, n, k, tile width, split-K (-1 = stream-K)}; regenerate with "
-                "`python -m radeonflow_kernels_b200.tune --emit-inc`.\n")
+                "`python -m radeonflow_kernels_b200.tune --emit-inc`.\n"
+                "// The times are a graph's of launches over operand sets in turn, a rested chip's: calls one after the other take "
+                "longer.\n")
         for (m, n, k, bn, s, us) in table:
             f.write(f"{{{m}, {n}, {k}, {bn}, {s}}},   // {us:.2f} us\n")
 

@@ -42,6 +42,18 @@ def test_builtin_table_covers_the_benchmark_shapes(rf_lib):
         assert bn in (128, 256, 512) and (1 <= s <= k // 128 or s == tune.STREAM_K)
 
 
+def test_cost_model_names_the_plans_of_the_table(rf_lib):
+    """... but two, where pairs and one-CTA tiles of 256 columns are within 5 % of each other."""
+    code = ("from tests.test_gemm_plans import _get; from radeonflow_kernels_b200 import _lib, tune; "
+            "print([_get(_lib.lib(), *s) for s in tune.BENCHMARK_SHAPES])")
+    res = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True,
+                         env=dict(os.environ, RF_FP8_GEMM_NO_BUILTIN_PLANS="1"))
+    assert res.returncode == 0, res.stderr
+    model = eval(res.stdout.strip().splitlines()[-1])
+    other = {s: (_get(rf_lib, *s), p) for s, p in zip(tune.BENCHMARK_SHAPES, model) if _get(rf_lib, *s) != p}
+    assert other == {(1024, 3072, 1536): ((512, 1), (256, 1)), (6144, 1536, 7168): ((256, 1), (512, 1))}
+
+
 def _plan_list():
     """Plans of shapes around the lines between one pass, split-K in clusters and split-K through memory."""
     from radeonflow_kernels_b200 import _lib
